@@ -90,11 +90,8 @@ int rsfm_precomp_sift4b_sqr_norm(uint32_t* sqrNorm, const void* desc4b, uint32_t
  * Each distinct image is widened to bytes in stream-ordered scratch (128 B per descriptor). */
 int rsfm_bf_match_4b(const rsfm_sift_bf_task* tasks, size_t nbTasks, cudaStream_t stream);
 
-/* Allocation-free rsfm_bf_match (no counterpart in the reference): same results, but the per-row
- * second-best scratch is a fixed 4 MiB device array instead of stream-ordered allocations, so no
- * call allocates device memory. At most 1 Mi query rows (sum of nbDescA) per call, else
- * RSFM_ERR_CAPACITY. The first call on a device looks up the array's address (make it before any
- * stream capture). All calls share the array: calls that overlap on the GPU race. */
+/* Allocation-free rsfm_bf_match (no counterpart in the reference): same results; no call allocates
+ * device memory. At most 1 Mi query rows (sum of nbDescA) per call, else RSFM_ERR_CAPACITY. */
 int rsfm_bf_match_noalloc(const rsfm_sift_bf_task* tasks, size_t nbTasks, cudaStream_t stream);
 
 /* Extended form of rsfm_bf_match (no reference counterpart for the extra outputs): also writes,
@@ -112,9 +109,9 @@ int rsfm_bf_match_ext(const rsfm_sift_bf_task* tasks, size_t nbTasks, uint32_t* 
  * tensor maps are encoded once. Options: 0 = automatic. */
 typedef struct rsfm_bf_plan rsfm_bf_plan;
 typedef struct rsfm_bf_plan_options {
-    uint32_t rowTiles;        /* 128-row tiles per work unit (1..8) */
-    uint32_t colBlocks;       /* 128-column blocks per work unit */
-    uint32_t epilogueGroups;  /* epilogue warpgroups per CTA: 2 or 4 */
+    uint32_t rowTiles;        /* work unit area rowTiles x colBlocks (1..8 each) in 128 x 128 tiles; */
+    uint32_t colBlocks;       /*   units are 256 rows high, so only the area matters */
+    uint32_t epilogueGroups;  /* kept for callers of earlier versions; has no effect */
     uint32_t useGraph;        /* capture the launches in a CUDA graph */
     uint32_t schedule;        /* unit order: 0 = pairs in the given order, 1 = largest pairs first */
 } rsfm_bf_plan_options;
@@ -124,8 +121,8 @@ int rsfm_bf_plan_create(const rsfm_sift_bf_task* tasks, size_t nbTasks, uint32_t
 int rsfm_bf_plan_launch(rsfm_bf_plan* plan, cudaStream_t stream);
 int rsfm_bf_plan_destroy(rsfm_bf_plan* plan);
 
-/* Autotuner for batched plans (no reference counterpart). Times candidate options (unit shape
- * rowTiles x colBlocks, epilogue warpgroups, schedule) on this batch: each candidate is a graph
+/* Autotuner for batched plans (no reference counterpart). Times candidate options (unit area
+ * rowTiles x colBlocks, schedule) on this batch: each candidate is a graph
  * plan launched once to warm up and `reps` times under CUDA events on `stream` (so the batch's
  * outputs are written as a side effect); returns the fastest in *best and its time per launch in
  * *bestMs. With cachePath non-NULL, choices are kept in that text file keyed by a signature of

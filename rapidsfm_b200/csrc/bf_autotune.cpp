@@ -1,10 +1,10 @@
 // Autotuner for batched brute-force plans (no reference counterpart).
 //
 // A batch of uneven pairs is matched by one persistent launch; how fast depends on the unit
-// shape (row tiles x column blocks per unit: fewer column publishes and unit boundaries vs. more
-// units to balance), the epilogue warpgroup count and the order in which CTAs take units. The tuner times a pruned
-// grid of candidates on the batch itself and keeps the winner in an optional text cache keyed by
-// a coarse signature of the batch, so later batches of the same kind skip the timing.
+// length (columns per unit: fewer row publishes and unit boundaries vs. more units to balance) and
+// the order in which CTAs take units. The tuner times the candidates on the batch itself and keeps
+// the winner in an optional text cache keyed by a coarse signature of the batch, so later batches
+// of the same kind skip the timing.
 #include "../../include/rsfm_b200.h"
 
 #include <cuda_runtime.h>
@@ -14,6 +14,7 @@
 #include <mutex>
 #include <sstream>
 #include <string>
+#include <utility>
 
 namespace {
 
@@ -117,20 +118,14 @@ extern "C" int rsfm_bf_plan_autotune(const rsfm_sift_bf_task* tasks, size_t nbTa
             win = o;
         }
     };
-    // Stage 1: unit shape with four epilogue warpgroups, largest pairs first.
-    for (uint32_t rt : {8u, 4u, 2u})
-        for (uint32_t cb : {8u, 4u, 2u, 1u}) {
-            if (st != RSFM_OK) break;
-            trial(rsfm_bf_plan_options{rt, cb, 4u, 1u, 1u});
-        }
-    // Stage 2: warpgroups and schedule around the best shape.
-    const rsfm_bf_plan_options shape = win;
-    for (uint32_t g : {2u, 4u})
-        for (uint32_t sc : {0u, 1u}) {
-            if (st != RSFM_OK) break;
-            if (g == shape.epilogueGroups && sc == shape.schedule) continue;
-            trial(rsfm_bf_plan_options{shape.rowTiles, shape.colBlocks, g, 1u, sc});
-        }
+    // Stage 1: unit length (units are 256 rows high; the options' area rowTiles x colBlocks gives
+    // 16, 8, 4, 2 or 1 blocks of 256 columns), largest pairs first.
+    for (const auto& sh : {std::pair<uint32_t, uint32_t>{8u, 8u}, {8u, 4u}, {8u, 2u}, {8u, 1u}, {4u, 1u}}) {
+        if (st != RSFM_OK) break;
+        trial(rsfm_bf_plan_options{sh.first, sh.second, 4u, 1u, 1u});
+    }
+    // Stage 2: the given pair order with the best length.
+    if (st == RSFM_OK) trial(rsfm_bf_plan_options{win.rowTiles, win.colBlocks, 4u, 1u, 0u});
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (st != RSFM_OK) return st;

@@ -17,10 +17,30 @@ constexpr int kMaxTasksPerLaunch = 16;
 // result alignment, and the per-task size limit (RSFM_ERR_CAPACITY above 0x7FFFFF00 rows).
 int validate(const rsfm_sift_bf_task* tasks, size_t n);
 
-// Init + matcher (+ flags when `flags` is non-null) for n <= kMaxTasksPerLaunch tasks on
-// `stream`; second[t] is task t's per-row second-best buffer (nbDescA entries).
+// Results of up to kMaxTasksPerLaunch tasks, as the kernel that initialises them gets them.
+struct InitParams {
+    unsigned long long* bestA[kMaxTasksPerLaunch];
+    unsigned long long* bestB[kMaxTasksPerLaunch];
+    uint32_t* secondA[kMaxTasksPerLaunch];  // null entries: no second-best output
+    uint32_t nA[kMaxTasksPerLaunch], nB[kMaxTasksPerLaunch];
+};
+inline InitParams init_params(const rsfm_sift_bf_task* tasks, size_t n, uint32_t* const* second) {
+    InitParams ip{};
+    for (size_t t = 0; t < n; ++t) {
+        ip.bestA[t] = reinterpret_cast<unsigned long long*>(tasks[t].bestMatchA);
+        ip.bestB[t] = reinterpret_cast<unsigned long long*>(tasks[t].bestMatchB);
+        ip.secondA[t] = second ? second[t] : nullptr;
+        ip.nA[t] = tasks[t].nbDescA;
+        ip.nB[t] = tasks[t].nbDescB;
+    }
+    return ip;
+}
+
+// Init + matcher + index resolution (+ flags when `flags` is non-null, which needs `second`) for
+// n <= kMaxTasksPerLaunch tasks on `stream`; second[t] is task t's per-row second-best output
+// (nbDescA entries), `second` may be null. initialised: the results already hold ~0 on `stream`.
 int launch_chunk(const rsfm_sift_bf_task* tasks, size_t n, uint32_t* const* second, uint32_t* const* flags,
-                 uint32_t ratioNum, uint32_t ratioDen, cudaStream_t stream);
+                 uint32_t ratioNum, uint32_t ratioDen, cudaStream_t stream, bool initialised = false);
 
 }  // namespace bf
 }  // namespace rsfm_b200

@@ -11,26 +11,42 @@
 // Extension (no reference counterpart): per A row the second-smallest distance, used by the
 // ratio test; flags for the ratio test and the cross-check.
 //
-// Work decomposition. A "unit" is a block of up to kMaxRowTiles*128 A rows times a range of up to
-// kMaxColBlocks 128-column B blocks. Persistent CTAs take units round-robin. Per CTA:
-//   warp 0      TMA producer: A row tiles (resident for the unit), B column blocks (ring)
-//   warp 1      TMEM allocator and UMMA issuer (one thread): per (B block, A row tile) two
-//               128x128x128 int8 products into one of two TMEM accumulator pairs: the tile
-//               (lane = A row, column = B column) and its transpose (lane = B column, column =
-//               A row), from the same shared-memory operands with their roles swapped
-//   warps 2..   epilogue, 2 or 4 warpgroups; warpgroup w owns 128/G columns of every tile and,
-//               in the transpose, the same number of rows
-// Both reductions are thread-local: from the tile an epilogue thread reads one A row (its row
-// minimum), from the transpose one B column over the warpgroup's row slice (its column minimum,
-// kept in a register across the unit's row tiles and published with one global atomic per B
-// block). The exact row second-best needs per-chunk work only for chunks that can still become
-// the row's best. Row state lives in shared memory per (warpgroup, row).
+// Every value that the epilogue compares leaves the tensor cores finished: an accumulator holds
+//   tile       (lane = A row i, column = B column j)   2 a_i.b_j - (|b_j|^2 - cB)
+//   transpose  (lane = B column j, column = A row i)   2 a_i.b_j - (|a_i|^2 - cA)
+// (cA, cB: norms of the unit's first row and column), i.e. the distance up to a constant of the
+// lane. The factor 2 comes from A tiles doubled in shared memory (bytes <= 127; a unit with a larger
+// byte keeps its bytes and issues every product twice), the norms from one more K = 32 step: a
+// constant operand [1, 127 x 15][1, 127 x 15] times per-descriptor s8 digits. A norm that the
+// digits do not reach, and rows or columns past the end, leave a residual that the epilogue adds
+// (slices that have one are flagged).
+//
+// The epilogue keeps, per lane, only maxima of 16-column chunks: one key (value << 8 | chunk
+// code) per chunk, the best (and for the second-best output the two best) in registers. Results
+// are published as (distance, first index of the chunk), the minimum over chunks being the
+// lexicographic (distance, chunk) minimum; a last phase (resolve_item) then finds the index inside the
+// winning chunk, and the second-best inside it, from 16 exact distances.
+//
+// What bounds it: the tensor pipe. At 32768 x 32768 the two products take 2 x 5 K steps of 138
+// cycles per 128 x 256 values = 155 us on 148 SMs; keys formed on the CUDA cores instead (two
+// multiply-adds and a trigger per distance, the design before this one) took 362 us at 53 % issue.
+//
+// Work decomposition. A "unit" is a block of 256 A rows times up to 32 blocks of 256 B columns.
+// Persistent CTAs take units round-robin. Per CTA (768 threads):
+//   warp 0      UMMA issuer (one thread; warp 1 owns the TMEM allocation, 2 and 3 are idle): per B
+//               block the tiles of both 128-row halves and the transposes of both 128-column
+//               halves, each M = 128, N = 256, into two pairs of accumulators (128 TMEM columns
+//               each) in turn
+//   warps 4-7   TMA loads (A rows of a unit into two slots: the next unit's load and are prepared
+//               during this one; B blocks into three stages), doubling of the A rows, digits,
+//               residuals, norms, unit description
+//   warps 8-23  epilogue: warpgroup g reads accumulator g, warp q of it TMEM lanes 32q..
 #include "bf_internal.h"
 #include "common.h"
 #include "sm100.cuh"
 #include <algorithm>
 #include <climits>
-#include <cstdlib>
+#include <cooperative_groups.h>
 #include <vector>
 
 namespace rsfm_b200 {
@@ -38,37 +54,34 @@ namespace bf {
 
 using namespace sm100;
 
-constexpr int kMaxRowTiles = 8;        // A row tiles per unit (p fits 3 bits of the keys)
-constexpr int kTileBytes = 128 * 128;  // 128 descriptors x 128 bytes
-constexpr int kUnitRows = kMaxRowTiles * 128;
-constexpr int kMaxColBlocks = 8;       // B blocks per unit
-constexpr int kUnitCols = kMaxColBlocks * 128;
-constexpr int kAccBufs = 2;            // TMEM accumulator pairs (all 512 columns)
-constexpr uint32_t kAccCols = 256;     // per pair: the 128 x 128 tile and its transpose
-// Epilogue warpgroups kWG in {2, 4}: warpgroup w owns 128/kWG columns of every tile, i.e.
-// kCPW = 4/kWG chunks of 32 columns per warp. Four warpgroups leave room for two B stages.
-template <int kWG>
-struct Cfg {
-    static constexpr int kEpiWarps = 4 * kWG;
-    static constexpr int kThreads = 32 * (2 + kEpiWarps);
-    static constexpr int kCPW = 4 / kWG;
-    static constexpr int kBStages = kWG == 4 ? 2 : 3;
-};
-constexpr uint32_t kMaxDist = 128u * 255u * 255u;  // largest possible squared L2 of uint8x128
-
+constexpr uint32_t kUnitRows = 256;      // A rows per unit (two 128-lane tiles)
+constexpr uint32_t kBlockCols = 256;     // B columns per block (two 128-lane transposes)
+constexpr uint32_t kChunk = 16;          // values per key
+constexpr int kBStages = 3;
+constexpr int kASlots = 2;
+constexpr uint32_t kPrepThreads = 128;
+constexpr uint32_t kEpiWarps = 16;
+constexpr uint32_t kThreads = 32 * (4 + kEpiWarps) + kPrepThreads;
+constexpr uint32_t kTileBytes = 256 * 128;
+constexpr uint32_t kDigitBytes = 256 * 32;
+constexpr int32_t kNoValue = -(1 << 23);  // below every 2ab - |x|^2 (> -128 * 255^2)
 
 struct alignas(64) TaskDev {
     CUtensorMap tmA;
     CUtensorMap tmB;
+    const uint4* descA;
+    const uint4* descB;
     const uint32_t* sqrA;
     const uint32_t* sqrB;
     unsigned long long* bestA;  // rsfm_best_match viewed as (distance << 32 | index)
     unsigned long long* bestB;
-    uint32_t* secondA;
-    uint32_t* flagsA;  // batched plans only (the per-call path passes flags separately)
+    uint32_t* secondA;  // null: no second-best output
+    uint32_t* flagsA;   // null: no flags
     uint32_t nA, nB;
-    uint32_t rowBlocks, colRanges;
-    uint32_t unitBegin;
+    uint32_t rowBlocks;
+    uint32_t unitBegin;   // first unit, first group of 4 results to resolve, first group of 32 rows:
+    uint32_t groupBegin;  // each in the order of the tasks
+    uint32_t rowGroupBegin;
 };
 
 struct Params {
@@ -76,64 +89,65 @@ struct Params {
     const TaskDev* gtasks;  // when non-null: any number of tasks, in global memory
     uint32_t nTasks;
     uint32_t totalUnits;
-    uint32_t rowTiles;  // row tiles per unit (<= kMaxRowTiles)
-    uint32_t colBlocks; // 128-column blocks per unit (<= kMaxColBlocks)
+    uint32_t totalGroups, totalRowGroups;  // totalRowGroups: 0 without flags
+    uint32_t ratioNum, ratioDen;
+    uint32_t fused;       // cooperative launch: the matcher also resolves and sets the flags
+    uint32_t unitBlocks;  // 256-column blocks per unit (<= 32: the chunk code holds 8 * 32 values)
     uint32_t* err;
 };
 
 struct Unit {
-    uint32_t task, r0, c0, pt, cb;
+    uint32_t r0, c0, rows, cols;
 };
 
 __device__ __forceinline__ const TaskDev& task_of(const Params& P, uint32_t t) {
     return P.gtasks ? P.gtasks[t] : P.tasks[t];
 }
 
-__device__ __forceinline__ Unit decode_unit(const Params& P, uint32_t u) {
-    uint32_t t = 0;
-    if (P.gtasks) {  // last task whose first unit is <= u
-        uint32_t lo = 0, hi = P.nTasks - 1;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi + 1) >> 1;
-            if (P.gtasks[mid].unitBegin <= u) lo = mid; else hi = mid - 1;
-        }
-        t = lo;
-        while (t + 1 < P.nTasks && P.gtasks[t + 1].unitBegin <= u) ++t;
-    } else {
-        while (t + 1 < P.nTasks && u >= P.tasks[t + 1].unitBegin) ++t;
-    }
+// Unit u of task t, where t enters as the task of an earlier unit of this CTA (units are taken in
+// increasing order, so the search only moves forward).
+__device__ __forceinline__ Unit decode_unit(const Params& P, uint32_t u, uint32_t& t) {
+    while (t + 1 < P.nTasks && task_of(P, t + 1).unitBegin <= u) ++t;
     const TaskDev& T = task_of(P, t);
     const uint32_t local = u - T.unitBegin;
     const uint32_t cr = local / T.rowBlocks;
-    const uint32_t rb = local - cr * T.rowBlocks;
     Unit U;
-    U.task = t;
-    U.r0 = rb * 128u * P.rowTiles;
-    U.c0 = cr * 128u * P.colBlocks;
-    uint32_t pt = (T.nA - U.r0 + 127u) / 128u;
-    U.pt = pt < P.rowTiles ? pt : P.rowTiles;
-    uint32_t cb = (T.nB - U.c0 + 127u) / 128u;
-    U.cb = cb < P.colBlocks ? cb : P.colBlocks;
+    U.r0 = (local - cr * T.rowBlocks) * kUnitRows;
+    U.c0 = cr * kBlockCols * P.unitBlocks;
+    U.rows = min(T.nA - U.r0, kUnitRows);
+    U.cols = min(T.nB - U.c0, kBlockCols * P.unitBlocks);
     return U;
 }
 
-template <int kWG>
+// What the issuer and the epilogue need to know about the unit in an A slot.
+struct UnitInfo {
+    unsigned long long* bestA;
+    unsigned long long* bestB;
+    uint32_t* secondA;
+    uint32_t r0, c0, rows, cols;
+    uint32_t cA, cB;  // norms of the first row and column
+    uint32_t big;     // some A byte exceeds 127: not doubled, products issued twice
+};
+
 struct Smem {
-    // A row tiles and B stages are 1024-byte aligned (128-byte swizzle atoms).
-    uint8_t a[kMaxRowTiles][kTileBytes];
-    uint8_t b[Cfg<kWG>::kBStages][kTileBytes];
-    int32_t nbk[kUnitCols];              // per unit column: row-key addend (31 - j % 32) - |b|^2 * 256
-    // Row state of the current unit, per unit row r = 128 p + 32 q + lane:
-    int32_t rowc[kUnitRows];             // column-key addend ((7-p) << 5 | (31-lane)) - |a|^2 * 256
-    // Per warpgroup: tk = trigger threshold in row-key space (set from the global best at unit
-    // start, tie-inclusive; after the warpgroup's own best d1 it is -(d1 - 1) * 256 + c, i.e.
-    // strictly better); l2k = second key; l1j = column of the own best (0xFFFF: none yet).
-    int32_t tk[kWG][kUnitRows];
-    int32_t l2k[kWG][kUnitRows];
-    uint16_t l1j[kWG][kUnitRows];
-    uint64_t aFull[kMaxRowTiles], aEmpty[kMaxRowTiles];
-    uint64_t bFull[Cfg<kWG>::kBStages], bEmpty[Cfg<kWG>::kBStages];
-    uint64_t accFull[kAccBufs], accEmpty[kAccBufs];
+    // A rows and B blocks: 128-byte rows, 128-byte swizzle (1024-byte atoms)
+    uint8_t a[kASlots][kTileBytes];
+    uint8_t b[kBStages][kTileBytes];
+    // norm digits: 32-byte rows, 32-byte swizzle (256-byte atoms)
+    uint8_t digA[kASlots][kDigitBytes];
+    uint8_t digB[kBStages][kDigitBytes];
+    uint8_t ones[128 * 32];
+    int32_t resA[kASlots][256];
+    int32_t resB[kBStages][256];
+    uint32_t nrmA[kASlots][256];
+    uint32_t nrmB[kBStages][256];
+    uint32_t flagA[kASlots][4];  // per 64-row slice: nonzero when some residual is
+    uint32_t flagB[kBStages][4];
+    UnitInfo info[kASlots];
+    uint32_t bigWarp[4];
+    uint64_t aRaw[kASlots], aReady[kASlots], aEpi[kASlots];
+    uint64_t bReady[kBStages], bEpi[kBStages];
+    uint64_t accFull[2], accEmpty[2];  // per pair of accumulators
     uint64_t mmaDone;
     uint32_t tmemBase;
 };
@@ -142,28 +156,198 @@ __device__ __forceinline__ void named_bar(uint32_t id, uint32_t n) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
 
-template <int kWG>
-__global__ void __launch_bounds__(Cfg<kWG>::kThreads, 1) bf_match_kernel(const __grid_constant__ Params P) {
-    constexpr int kEpiWarps = Cfg<kWG>::kEpiWarps;
-    constexpr int kCPW = Cfg<kWG>::kCPW;
-    constexpr int kBStages = Cfg<kWG>::kBStages;
+// s8 digits of w for the constant operand (row r of a 32-byte swizzled tile): d0 + 127 Q, Q spread
+// over 30 digits; |w| <= 127 * 3810 + 63 is exact. Returns what is left.
+__device__ __forceinline__ int32_t store_digits(uint8_t* tile, uint32_t r, int32_t w) {
+    constexpr int32_t kQmax = 30 * 127;
+    int32_t Q = __float2int_rn(float(w) * (1.f / 127.f));
+    int32_t d0 = w - 127 * Q, left = 0;
+    uint32_t dg[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (uint32_t(Q + 127) <= 254u) {  // one digit holds Q: norms within 16 K of each other
+        dg[0] = (uint32_t(Q) & 255u) << 8;
+    } else {
+        Q = max(-kQmax, min(kQmax, Q));
+        d0 = max(-127, min(127, w - 127 * Q));
+        left = w - d0 - 127 * Q;
+#pragma unroll
+        for (int k = 1; k < 32; ++k) {
+            if (k == 16) continue;  // the other weight-1 slot stays 0
+            const int32_t v = max(-127, min(127, Q));
+            dg[k >> 2] |= (uint32_t(v) & 255u) << (8 * (k & 3));
+            Q -= v;
+        }
+    }
+    dg[0] |= uint32_t(d0) & 255u;
+    const uint32_t swap = ((r >> 2) & 1u) << 4;
+    uint8_t* row = tile + 32u * r;
+    *reinterpret_cast<uint4*>(row + swap) = make_uint4(dg[0], dg[1], dg[2], dg[3]);
+    *reinterpret_cast<uint4*>(row + (16u ^ swap)) = make_uint4(dg[4], dg[5], dg[6], dg[7]);
+    return left;
+}
+
+// Maxima of the two 16-value chunks of x, as four chains (a chain of eight 3-input maxima is
+// latency-bound).
+__device__ __forceinline__ void chunk_max(const uint32_t (&x)[32], int32_t& m0, int32_t& m1) {
+    int32_t m[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) m[c] = __vimax3_s32(int32_t(x[8 * c]), int32_t(x[8 * c + 1]), int32_t(x[8 * c + 2]));
+#pragma unroll
+    for (int k = 3; k < 7; k += 2)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) m[c] = __vimax3_s32(m[c], int32_t(x[8 * c + k]), int32_t(x[8 * c + k + 1]));
+    m0 = __vimax3_s32(max(m[0], int32_t(x[7])), m[1], int32_t(x[15]));
+    m1 = __vimax3_s32(max(m[2], int32_t(x[23])), m[3], int32_t(x[31]));
+}
+
+__device__ __forceinline__ void add_residuals(uint32_t (&x)[32], const int32_t* res) {
+    const int4* r4 = reinterpret_cast<const int4*>(res);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int4 r = r4[k];
+        x[4 * k] += uint32_t(r.x);
+        x[4 * k + 1] += uint32_t(r.y);
+        x[4 * k + 2] += uint32_t(r.z);
+        x[4 * k + 3] += uint32_t(r.w);
+    }
+}
+
+// ---------------------------------------------------------------- index inside the winning chunk
+// The matcher leaves (distance, first index of a 16-descriptor chunk) per row and per column; eight
+// lanes per item compute the chunk's 16 exact distances (each lane 16 bytes of every descriptor:
+// one cache line per descriptor) and keep the first index at that distance. With `second`, the
+// chunk's other distances complete the second-best. Bound by L2 reads, 2 KiB per item: 134 MB for
+// 32768 x 32768; chunks of 32 values would save the matcher 4 of 48 operations per 64 values and
+// double these reads.
+__device__ __forceinline__ void resolve_item(const uint4* __restrict__ q, const uint4* __restrict__ set, uint32_t nSet,
+                                             uint32_t normQ, const uint32_t* __restrict__ sqrSet,
+                                             unsigned long long* best, uint32_t* second, bool in, uint32_t l8) {
+    const unsigned long long bst = in ? __ldcg(best) : ~0ull;
+    const uint32_t j0 = uint32_t(bst), d = uint32_t(bst >> 32);
+    const bool has = in && j0 != ~0u;
+    uint32_t dot[kChunk];
+    uint4 qv = make_uint4(0, 0, 0, 0), tv[kChunk];
+    if (has) qv = __ldg(&q[l8]);
+#pragma unroll
+    for (uint32_t k = 0; k < kChunk; ++k) {
+        tv[k] = make_uint4(0, 0, 0, 0);
+        if (has && j0 + k < nSet) tv[k] = __ldg(&set[size_t(j0 + k) * 8 + l8]);
+    }
+    // this lane ends up with the sums of candidates 2 * l8 and 2 * l8 + 1
+    uint32_t nv[2] = {0, 0};
+#pragma unroll
+    for (uint32_t e = 0; e < 2; ++e)
+        if (has && j0 + 2 * l8 + e < nSet) nv[e] = __ldg(&sqrSet[j0 + 2 * l8 + e]);
+#pragma unroll
+    for (uint32_t k = 0; k < kChunk; ++k) {
+        uint32_t a = __dp4a(qv.x, tv[k].x, 0u);
+        a = __dp4a(qv.y, tv[k].y, a);
+        a = __dp4a(qv.z, tv[k].z, a);
+        dot[k] = __dp4a(qv.w, tv[k].w, a);
+    }
+#pragma unroll
+    for (uint32_t w = 8; w >= 2; w >>= 1) {  // halve the candidates, add the partner's half
+        const uint32_t o = w >> 1;           // lane distance 4, 2, 1
+        const bool hi = (l8 & o) != 0u;
+#pragma unroll
+        for (uint32_t k = 0; k < w; ++k) {
+            const uint32_t mine = hi ? dot[k + w] : dot[k], theirs = hi ? dot[k] : dot[k + w];
+            dot[k] = mine + __shfl_xor_sync(0xffffffffu, theirs, o);
+        }
+    }
+    uint32_t dist[2], at = ~0u;
+#pragma unroll
+    for (int e = 1; e >= 0; --e) {
+        const uint32_t j = j0 + 2 * l8 + e;
+        dist[e] = has && j < nSet ? normQ + nv[e] - 2u * dot[e] : ~0u;
+        if (has && j < nSet && dist[e] == d) at = j;
+    }
+#pragma unroll
+    for (uint32_t o = 1; o < 8; o <<= 1) at = min(at, __shfl_xor_sync(0xffffffffu, at, o));
+    uint32_t s = ~0u;  // (shuffled by every lane: rows and columns may share a warp)
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+        if (j0 + 2 * l8 + e != at) s = min(s, dist[e]);
+#pragma unroll
+    for (uint32_t o = 1; o < 8; o <<= 1) s = min(s, __shfl_xor_sync(0xffffffffu, s, o));
+    if (second && has && l8 == 0 && s < __ldcg(second)) *second = s;
+    if (has && l8 == 0 && at != ~0u) *best = (static_cast<unsigned long long>(d) << 32) | at;
+}
+
+// Last task at or after t whose `begin` is <= w (tasks without any share their successor's).
+__device__ __forceinline__ uint32_t task_at(const Params& P, uint32_t t, uint32_t TaskDev::*begin, uint32_t w) {
+    uint32_t hi = P.nTasks - 1u;
+    while (t < hi) {
+        const uint32_t mid = (t + hi + 1u) >> 1;
+        if (task_of(P, mid).*begin <= w) t = mid; else hi = mid - 1u;
+    }
+    return t;
+}
+
+// Warp w0 of `warps` takes a run of consecutive groups of four results (rows of A, then columns of
+// B), eight lanes a result.
+__device__ __forceinline__ void resolve_phase(const Params& P, uint32_t w0, uint32_t warps, uint32_t lane) {
+    const uint32_t l8 = lane & 7u;
+    uint32_t t = 0;
+    const uint32_t run = (P.totalGroups + warps - 1u) / warps, first = w0 * run;
+    const uint32_t end = first < P.totalGroups ? min(P.totalGroups, first + run) : first;
+    if (first < end) t = task_at(P, 0u, &TaskDev::groupBegin, first);
+    for (uint32_t w = first; w < end; ++w) {
+        while (t + 1 < P.nTasks && task_of(P, t + 1).groupBegin <= w) ++t;
+        const TaskDev& T = task_of(P, t);
+        const uint64_t x = uint64_t(w - T.groupBegin) * 4u + (lane >> 3);
+        const bool row = x < T.nA, in = x < uint64_t(T.nA) + T.nB;
+        const uint32_t i = row ? uint32_t(x) : in ? uint32_t(x - T.nA) : 0u;
+        const uint4* q = (row ? T.descA : T.descB) + size_t(i) * 8;
+        const uint32_t nq = in ? __ldg((row ? T.sqrA : T.sqrB) + i) : 0u;
+        resolve_item(q, row ? T.descB : T.descA, row ? T.nB : T.nA, nq, row ? T.sqrB : T.sqrA,
+                     (row ? T.bestA : T.bestB) + i, row && T.secondA ? T.secondA + i : nullptr, in, l8);
+    }
+}
+
+// Flags of every row: bit0 ratio test, bit1 cross-check. Runs of 32-row groups as above.
+__device__ __forceinline__ void flags_phase(const Params& P, uint32_t w0, uint32_t warps, uint32_t lane) {
+    uint32_t t = 0;
+    const uint32_t run = (P.totalRowGroups + warps - 1u) / warps, first = w0 * run;
+    const uint32_t end = first < P.totalRowGroups ? min(P.totalRowGroups, first + run) : first;
+    if (first < end) t = task_at(P, 0u, &TaskDev::rowGroupBegin, first);
+    for (uint32_t w = first; w < end; ++w) {
+        while (t + 1 < P.nTasks && task_of(P, t + 1).rowGroupBegin <= w) ++t;
+        const TaskDev& T = task_of(P, t);
+        const uint32_t i = (w - T.rowGroupBegin) * 32u + lane;
+        if (i >= T.nA) continue;
+        const unsigned long long bm = __ldcg(&T.bestA[i]);
+        const uint32_t j = uint32_t(bm & 0xFFFFFFFFu), d = uint32_t(bm >> 32);
+        uint32_t f = 0;
+        if (j != ~0u) {
+            if (uint64_t(P.ratioDen) * d < uint64_t(P.ratioNum) * __ldcg(&T.secondA[i])) f |= 1u;
+            if (j < T.nB && uint32_t(__ldcg(&T.bestB[j]) & 0xFFFFFFFFu) == i) f |= 2u;
+        }
+        T.flagsA[i] = f;
+    }
+}
+
+// kSecond: the second-best distances are wanted too.
+template <bool kSecond>
+__global__ void __launch_bounds__(kThreads, 1) bf_match_kernel(const __grid_constant__ Params P) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    Smem<kWG>& S = smem_aligned_1024<Smem<kWG>>(smem_raw);
+    Smem& S = smem_aligned_1024<Smem>(smem_raw);
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31u;
 
     if (threadIdx.x == 0) {
-        for (int p = 0; p < kMaxRowTiles; ++p) {
-            mbar_init(&S.aFull[p], 1);
-            mbar_init(&S.aEmpty[p], 1);
+        for (int s = 0; s < kASlots; ++s) {
+            S.info[s].rows = S.info[s].cols = 0;  // a timed-out wait must find nothing to write
+            mbar_init(&S.aRaw[s], 1);
+            mbar_init(&S.aReady[s], kPrepThreads);
+            mbar_init(&S.aEpi[s], kEpiWarps);
         }
         for (int s = 0; s < kBStages; ++s) {
-            mbar_init(&S.bFull[s], 1);
-            mbar_init(&S.bEmpty[s], 1);
+            mbar_init(&S.bReady[s], kPrepThreads);  // (and the bytes of the TMA load)
+            mbar_init(&S.bEpi[s], kEpiWarps);
         }
-        for (int s = 0; s < kAccBufs; ++s) {
+        for (uint32_t s = 0; s < 2; ++s) {
             mbar_init(&S.accFull[s], 1);
-            mbar_init(&S.accEmpty[s], kEpiWarps);
+            mbar_init(&S.accEmpty[s], kEpiWarps / 2);
         }
         mbar_init(&S.mmaDone, 1);
         fence_mbar_init();
@@ -172,366 +356,337 @@ __global__ void __launch_bounds__(Cfg<kWG>::kThreads, 1) bf_match_kernel(const _
         tmem_alloc(&S.tmemBase, 512);
         tmem_relinquish();
     }
+    if (threadIdx.x >= 128 && threadIdx.x < 384) {  // 128 x 32 bytes; both 16-byte chunks alike
+        reinterpret_cast<uint4*>(S.ones)[threadIdx.x - 128] =
+            make_uint4(0x7F7F7F01u, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu);
+        fence_proxy_async_smem();
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = S.tmemBase;
     uint32_t* err = P.err;
 
-    if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer
-        if (elect_one()) {
-            uint32_t aUse = 0;  // bit p: parity of loads issued into A slot p
-            uint32_t stage = 0, bPhase = 0;
-            auto loadA = [&](const Unit& U) {
-                const TaskDev& T = task_of(P, U.task);
-                for (uint32_t p = 0; p < U.pt; ++p) {
-                    const uint32_t par = ((aUse >> p) & 1u) ^ 1u;
-                    mbar_wait(&S.aEmpty[p], par, err, kDevTimeoutTmaEmpty);
-                    mbar_arrive_expect_tx(&S.aFull[p], kTileBytes);
-                    tma_load_2d(S.a[p], &T.tmA, &S.aFull[p], 0, int32_t(U.r0 + 128u * p));
-                    aUse ^= 1u << p;
-                }
-            };
-            uint32_t u = blockIdx.x;
-            if (u < P.totalUnits) {
-                const Unit U0 = decode_unit(P, u);
-                tma_prefetch_desc(&task_of(P, U0.task).tmA);
-                tma_prefetch_desc(&task_of(P, U0.task).tmB);
-                loadA(U0);
-            }
-            for (; u < P.totalUnits; u += gridDim.x) {
-                const Unit U = decode_unit(P, u);
-                const TaskDev& T = task_of(P, U.task);
-                for (uint32_t b = 0; b < U.cb; ++b) {
-                    mbar_wait(&S.bEmpty[stage], bPhase ^ 1u, err, kDevTimeoutTmaEmpty);
-                    mbar_arrive_expect_tx(&S.bFull[stage], kTileBytes);
-                    tma_load_2d(S.b[stage], &T.tmB, &S.bFull[stage], 0, int32_t(U.c0 + 128u * b));
-                    if (++stage == uint32_t(kBStages)) { stage = 0; bPhase ^= 1u; }
-                }
-                const uint32_t un = u + gridDim.x;
-                if (un < P.totalUnits) loadA(decode_unit(P, un));
-            }
-        }
-    } else if (warp == 1) {
+    // Registers: 768 threads x 80 at launch = 40 + 56 + 4 x 96 per thread of the six warpgroups.
+    if (warp < 4) {
         // ------------------------------------------------------------ UMMA issuer
-        if (elect_one()) {
-            const uint32_t idesc = idesc_u8u8_s32(128, 128);
-            const uint64_t aDesc0 = umma_desc_k_sw128(smem_u32(S.a[0]));
-            uint32_t aUse = 0, stage = 0, bPhase = 0, acc = 0;
-            for (uint32_t u = blockIdx.x; u < P.totalUnits; u += gridDim.x) {
-                const Unit U = decode_unit(P, u);
-                for (uint32_t b = 0; b < U.cb; ++b) {
-                    mbar_wait(&S.bFull[stage], bPhase, err, kDevTimeoutTmaFull);
-                    const uint64_t bDesc = umma_desc_k_sw128(smem_u32(S.b[stage]));
-                    for (uint32_t p = 0; p < U.pt; ++p) {
-                        if (b == 0) {
-                            mbar_wait(&S.aFull[p], (aUse >> p) & 1u, err, kDevTimeoutTmaFull);
-                            aUse ^= 1u << p;
-                        }
-                        const uint32_t buf = acc % kAccBufs;
-                        mbar_wait(&S.accEmpty[buf], ((acc / kAccBufs) & 1u) ^ 1u, err, kDevTimeoutAccEmpty);
-                        tc_fence_after();
-                        // K step k = +32 bytes = +2 in the descriptor's start-address field (the
-                        // tiles sit below 256 KB, so the 14-bit field cannot carry).
-                        const uint64_t aDesc = aDesc0 + uint64_t(p) * (kTileBytes >> 4);
-                        // tile (rows x columns) and its transpose (columns x rows), side by side
-                        const uint32_t d = tmem + buf * kAccCols;
+        // One thread, so that products complete in order (with two or four issuers their UMMAs take
+        // turns, all accumulators fill at the same time and the epilogue runs in bursts: 294 and
+        // 335 us at 32768 x 32768); N = 256, because N = 128 reads 128 bytes of shared memory a
+        // cycle, all there is.
+        if (warp == 0 && elect_one()) {
+            const uint32_t idesc = idesc_u8u8_s32(128, 256), idescN = idesc | (1u << 7) | (1u << 10);  // s8 digits
+            constexpr uint32_t kHalf = 128u * 128u >> 4;  // descriptor step of 128 rows
+            const uint64_t ones = umma_desc_k_sw32(smem_u32(S.ones));
+            uint32_t stage = 0, bPhase = 0, use0 = 1, use1 = 1, k = 0;
+            for (uint32_t u = blockIdx.x; u < P.totalUnits; u += gridDim.x, ++k) {
+                const uint32_t slot = k & 1u;
+                mbar_wait(&S.aReady[slot], (k >> 1) & 1u, err, kDevTimeoutTmaFull);
+                const uint32_t cols = S.info[slot].cols, big = S.info[slot].big;
+                const bool two = S.info[slot].rows > 128u;
+                const uint64_t aDesc = umma_desc_k_sw128(smem_u32(S.a[slot]));
+                const uint64_t aDig = umma_desc_k_sw32(smem_u32(S.digA[slot]));
+                // a pair of accumulators: lanes x columns (4 K steps of 32 bytes = +2 in the
+                // start-address field), then the norms
+                auto product = [&](uint32_t pair, uint32_t& use, uint64_t lanes, uint64_t columns, uint64_t digits) {
+                    mbar_wait(&S.accEmpty[pair], use, err, kDevTimeoutAccEmpty);
+                    use ^= 1u;
+                    tc_fence_after();
+                    const uint32_t d = tmem + pair * 256u;
 #pragma unroll
-                        for (uint32_t k = 0; k < 4; ++k) umma_i8(d, aDesc + 2u * k, bDesc + 2u * k, idesc, k);
+                    for (uint32_t s = 0; s < 4; ++s) umma_i8(d, lanes + 2u * s, columns + 2u * s, idesc, s);
+                    if (big) {
 #pragma unroll
-                        for (uint32_t k = 0; k < 4; ++k) umma_i8(d + 128u, bDesc + 2u * k, aDesc + 2u * k, idesc, k);
-                        umma_commit(&S.accFull[buf]);
-                        if (b + 1 == U.cb) umma_commit(&S.aEmpty[p]);
-                        ++acc;
+                        for (uint32_t s = 0; s < 4; ++s) umma_i8(d, lanes + 2u * s, columns + 2u * s, idesc, 1u);
                     }
-                    umma_commit(&S.bEmpty[stage]);
+                    umma_i8(d, ones, digits, idescN, 1u);
+                    umma_commit(&S.accFull[pair]);
+                };
+                for (uint32_t c = 0; c < cols; c += kBlockCols) {
+                    mbar_wait(&S.bReady[stage], bPhase, err, kDevTimeoutTmaFull);
+                    tc_fence_after();
+                    const uint64_t bDesc = umma_desc_k_sw128(smem_u32(S.b[stage]));
+                    const uint64_t bDig = umma_desc_k_sw32(smem_u32(S.digB[stage]));
+                    product(0, use0, aDesc, bDesc, bDig);
+                    if (two) product(1, use1, aDesc + kHalf, bDesc, bDig);
+                    product(0, use0, bDesc, aDesc, aDig);
+                    if (cols - c > 128u) product(1, use1, bDesc + kHalf, aDesc, aDig);
                     if (++stage == uint32_t(kBStages)) { stage = 0; bPhase ^= 1u; }
                 }
             }
-            // Drain: every commit issued above has arrived once this one has.
+            // Drain: every product issued above is complete once this has arrived.
             umma_commit(&S.mmaDone);
             mbar_wait(&S.mmaDone, 0, err, kDevTimeoutOther);
         }
+    } else if (warp < 8) {
+        // ------------------------------------------------------------ loads and preparation
+        const uint32_t pt = threadIdx.x - 128u, pw = warp - 4u;
+        const uint32_t row0 = 64u * pw + lane;  // this thread's rows: row0, row0 + 32 (slice pw)
+        uint32_t stage = 0, bPhase = 0, k = 0, t = 0;
+        // 256 norms -> digits, residuals, norms, flags
+        auto digits = [&](const uint32_t (&nv)[2], uint32_t valid, uint32_t centre, uint8_t* tile, int32_t* res,
+                          uint32_t* nrm, uint32_t* flag) {
+            int32_t any = 0;
+#pragma unroll
+            for (uint32_t m = 0; m < 2; ++m) {
+                const uint32_t r = row0 + 32u * m;
+                const bool in = r < valid;
+                int32_t left = store_digits(tile, r, in ? int32_t(centre - nv[m]) : 0);
+                if (!in) left = int32_t(centre) + kNoValue;  // the descriptor reads as zero
+                res[r] = left;
+                nrm[r] = nv[m];
+                any |= left;
+            }
+            const uint32_t f = __any_sync(0xffffffffu, any != 0);
+            if (lane == 0) flag[pw] = f;
+        };
+        // norms [first, first + valid) of the slice, 0 past the end
+        auto norms = [&](uint32_t (&nv)[2], const uint32_t* sqr, uint32_t first, uint32_t valid) {
+#pragma unroll
+            for (uint32_t m = 0; m < 2; ++m) nv[m] = row0 + 32u * m < valid ? __ldg(&sqr[first + row0 + 32u * m]) : 0u;
+        };
+        // One thread issues the TMA loads; the stage or slot is free when the epilogue is done with
+        // its last use (which implies the products that read it are complete).
+        auto loadB = [&](const CUtensorMap* tm, uint32_t c, uint32_t st) {
+            mbar_expect_tx(&S.bReady[st], kTileBytes);
+            tma_load_2d(S.b[st], tm, &S.bReady[st], 0, int32_t(c));
+        };
+        auto loadA = [&](uint32_t u, uint32_t kk) {
+            uint32_t tn = t;
+            const Unit U = decode_unit(P, u, tn);
+            mbar_wait(&S.aEpi[kk & 1u], ((kk >> 1) & 1u) ^ 1u, err, kDevTimeoutTmaEmpty);
+            mbar_arrive_expect_tx(&S.aRaw[kk & 1u], kTileBytes);
+            tma_load_2d(S.a[kk & 1u], &task_of(P, tn).tmA, &S.aRaw[kk & 1u], 0, int32_t(U.r0));
+        };
+        auto prepA = [&](uint32_t u, uint32_t kk) {
+            const Unit U = decode_unit(P, u, t);
+            const TaskDev& T = task_of(P, t);
+            const uint32_t slot = kk & 1u, ph = (kk >> 1) & 1u;
+            uint32_t nv[2];
+            norms(nv, T.sqrA, U.r0, U.rows);
+            const uint32_t cA = __ldg(&T.sqrA[U.r0]), cB = __ldg(&T.sqrB[U.c0]);
+            mbar_wait(&S.aEpi[slot], ph ^ 1u, err, kDevTimeoutTmaEmpty);
+            digits(nv, U.rows, cA, S.digA[slot], S.resA[slot], S.nrmA[slot], S.flagA[slot]);
+            mbar_wait(&S.aRaw[slot], ph, err, kDevTimeoutTmaFull);
+            uint4* a4 = reinterpret_cast<uint4*>(S.a[slot]);
+            uint32_t any = 0;
+#pragma unroll 4
+            for (uint32_t x = pt; x < kTileBytes / 16; x += kPrepThreads) {
+                const uint4 v = a4[x];
+                any |= v.x | v.y | v.z | v.w;
+            }
+            any = __any_sync(0xffffffffu, (any & 0x80808080u) != 0u);
+            if (lane == 0) S.bigWarp[pw] = any;
+            named_bar(2, kPrepThreads);
+            const uint32_t big = S.bigWarp[0] | S.bigWarp[1] | S.bigWarp[2] | S.bigWarp[3];
+            if (!big) {
+#pragma unroll 4
+                for (uint32_t x = pt; x < kTileBytes / 16; x += kPrepThreads) {
+                    uint4 v = a4[x];
+                    v.x <<= 1;  // bytes <= 127: no carry into the next byte
+                    v.y <<= 1;
+                    v.z <<= 1;
+                    v.w <<= 1;
+                    a4[x] = v;
+                }
+            }
+            if (pt == 0) {
+                UnitInfo& I = S.info[slot];
+                I.bestA = T.bestA;
+                I.bestB = T.bestB;
+                I.secondA = T.secondA;
+                I.r0 = U.r0;
+                I.c0 = U.c0;
+                I.rows = U.rows;
+                I.cols = U.cols;
+                I.cA = cA;
+                I.cB = cB;
+                I.big = big;
+            }
+            fence_proxy_async_smem();
+            mbar_arrive(&S.aReady[slot]);
+            named_bar(2, kPrepThreads);  // bigWarp may be rewritten
+        };
+        uint32_t u = blockIdx.x;
+        uint32_t ahead = 0;  // blocks of the current unit whose loads are already under way
+        if (u < P.totalUnits) {
+            const Unit U = decode_unit(P, u, t);
+            ahead = min((U.cols + kBlockCols - 1) / kBlockCols, uint32_t(kBStages));
+            if (pt == 0) {
+                loadA(u, 0);
+                for (uint32_t b = 0; b < ahead; ++b) loadB(&task_of(P, t).tmB, U.c0 + kBlockCols * b, b);
+            }
+            prepA(u, 0);
+        }
+        for (; u < P.totalUnits; u += gridDim.x, ++k, ahead = 0) {
+            uint32_t tb = t;
+            const Unit U = decode_unit(P, u, tb);
+            const uint32_t* sqrB = task_of(P, tb).sqrB;
+            const CUtensorMap* tmB = &task_of(P, tb).tmB;
+            const uint32_t cB = __ldg(&sqrB[U.c0]);
+            const uint32_t nb = (U.cols + kBlockCols - 1) / kBlockCols;
+            const bool more = u + gridDim.x < P.totalUnits;
+            uint32_t nv[2], next[2];
+            norms(nv, sqrB, U.c0, U.cols);
+            for (uint32_t b = 0; b < nb; ++b) {
+                const uint32_t done = kBlockCols * (b + 1);
+                norms(next, sqrB, U.c0 + done, done < U.cols ? U.cols - done : 0u);
+                mbar_wait(&S.bEpi[stage], bPhase ^ 1u, err, kDevTimeoutTmaEmpty);
+                if (pt == 0 && b >= ahead) loadB(tmB, U.c0 + done - kBlockCols, stage);
+                digits(nv, U.cols - (done - kBlockCols), cB, S.digB[stage], S.resB[stage], S.nrmB[stage], S.flagB[stage]);
+                nv[0] = next[0];
+                nv[1] = next[1];
+                fence_proxy_async_smem();
+                mbar_arrive(&S.bReady[stage]);
+                if (++stage == uint32_t(kBStages)) { stage = 0; bPhase ^= 1u; }
+                // The next unit's rows: their slot is free from this unit's block 3 on (block 0 is done
+                // then, so the unit before is), and they have a block's time to arrive.
+                if (more && b == min(nb - 1, 3u) && pt == 0) loadA(u + gridDim.x, k + 1);
+                if (more && b == min(nb - 1, 4u)) prepA(u + gridDim.x, k + 1);
+            }
+        }
     } else {
         // ------------------------------------------------------------ epilogue
-        // Keys are kept in "max is better" form. For row 128 p + 32 m + l of a unit let
-        //   c = (7 - p) << 5 | (31 - l)                    (8 bits)
-        //   rowc = c - |a|^2 * 256                         (staged per unit row)
-        //   column key  ck = (2 a.b - |a|^2) * 256 + c     = (dot << 9) + rowc
-        //   row key     rk = ck + (31 - k) - |b|^2 * 256   = -d * 256 + c + (31 - k)
-        // (k = column within the 32-column chunk). A column's maximum ck over the rows of one
-        // 32-row slice (fixed m, any p and l) is its smallest d, ties going to the smallest row.
-        // Within one row c is constant and c + (31 - k) < 287, so row keys of one chunk order by
-        // (d, k); u = rk - c = -d * 256 + (31 - k) decodes both.
-        //
-        // Row state lives in shared memory, per warpgroup and unit row: tk = trigger threshold,
-        // l1j = column of the own best, l2k = max over the other keys that can matter for the
-        // second-best. A chunk does extra work only if its maximum reaches tk: it beats this
-        // warpgroup's best AND can still tie or beat the global best known at unit start; every
-        // other chunk contributes its maximum to l2k only. This is exact: a chunk that cannot
-        // hold the best holds at most one value that matters, its maximum.
-        const uint32_t e = warp - 2u;                    // epilogue warp
-        const uint32_t wg = e >> 2;                      // warpgroup: columns [32 kCPW wg, +32 kCPW)
-        const uint32_t q = warp & 3u;                    // TMEM lane quarter
-        const uint32_t tE = e * 32u + lane;              // 0 .. 32 kEpiWarps - 1
-        const uint32_t t128 = q * 32u + lane;            // row within a tile
-        const uint32_t laneBase = (32u * q) << 16;
-        constexpr int kRowIt = kUnitRows / (32 * kEpiWarps);
-        constexpr int kColIt = (kUnitCols + 32 * kEpiWarps - 1) / (32 * kEpiWarps);
-        uint32_t acc = 0;
-        for (uint32_t u = blockIdx.x; u < P.totalUnits; u += gridDim.x) {
-            const Unit U = decode_unit(P, u);
-            const TaskDev& T = task_of(P, U.task);
-            // ---- unit start: row state, row hints, column addends (all loads issued together)
-            uint32_t na[kRowIt], h1[kRowIt], nb[kColIt];
-#pragma unroll
-            for (int it = 0; it < kRowIt; ++it) {
-                const uint32_t r = tE + uint32_t(it) * 32u * kEpiWarps;
-                const uint32_t i = U.r0 + r;
-                const bool valid = (r >> 7) < U.pt && i < T.nA;
-                na[it] = valid ? __ldg(&T.sqrA[i]) : 0u;
-                h1[it] = valid ? uint32_t(__ldcg(&T.bestA[i]) >> 32) : kMaxDist;
-            }
-#pragma unroll
-            for (int it = 0; it < kColIt; ++it) {
-                const uint32_t x = tE + uint32_t(it) * 32u * kEpiWarps;
-                const uint32_t j = U.c0 + x;
-                nb[it] = (x < 128u * U.cb && j < T.nB) ? __ldg(&T.sqrB[j]) : 0u;
-            }
-#pragma unroll
-            for (int it = 0; it < kRowIt; ++it) {
-                const uint32_t r = tE + uint32_t(it) * 32u * kEpiWarps;
-                const uint32_t p = r >> 7, ln = r & 31u;
-                const uint32_t c = ((7u - p) << 5) | (31u - ln);
-                const uint32_t i = U.r0 + r;
-                const bool valid = p < U.pt && i < T.nA;
-                S.rowc[r] = valid ? int32_t(c - (na[it] << 8)) : int32_t(0x80000000u | c);
-                const int32_t t0 = valid ? int32_t((0u - (min(h1[it], kMaxDist) << 8)) + c) : INT32_MAX;
-#pragma unroll
-                for (int w = 0; w < kWG; ++w) {
-                    S.tk[w][r] = t0;
-                    S.l2k[w][r] = INT32_MIN;
-                    S.l1j[w][r] = 0xFFFFu;
+        // Warpgroup g owns accumulator g: per block the tile (row half g / 2, column half g % 2) and
+        // the transpose (column half g / 2, row half g % 2).
+        const uint32_t g = (warp - 8u) >> 2, q = warp & 3u;  // q: TMEM lane quarter
+        const uint32_t outer = 128u * (g >> 1), inner = 128u * (g & 1u);
+        const uint32_t mine = outer + 32u * q + lane;  // this thread's row (tile) or column (transpose)
+        const uint32_t taddr = tmem + ((32u * q) << 16) + 128u * g;
+        uint32_t accPhase = 0, stage = 0, bPhase = 0, k = 0;
+        // The accumulator's eight 16-value chunks as keys (value << 8) + base - chunk, handed to
+        // `take` in pairs.
+        auto chunks = [&](const int32_t* res, uint32_t base, auto&& take) {
+            mbar_wait(&S.accFull[g >> 1], accPhase, err, kDevTimeoutAccFull);
+            accPhase ^= 1u;
+            tc_fence_after();
+#pragma unroll 4
+            for (uint32_t part = 0; part < 4; ++part) {
+                uint32_t x[32];
+                tmem_ld16(taddr + 32u * part, *reinterpret_cast<uint32_t(*)[16]>(&x[0]));
+                tmem_ld16(taddr + 32u * part + 16u, *reinterpret_cast<uint32_t(*)[16]>(&x[16]));
+                tmem_wait_ld();
+                if (part == 3) {  // the accumulator is read: hand it back
+                    tc_fence_before();
+                    if (lane == 0) mbar_arrive(&S.accEmpty[g >> 1]);
                 }
+                if (res) add_residuals(x, res + 32u * part);
+                int32_t m0, m1;
+                chunk_max(x, m0, m1);
+                take(int32_t((uint32_t(m0) << 8) + (base - 2u * part)), int32_t((uint32_t(m1) << 8) + (base - 2u * part - 1u)));
             }
-#pragma unroll
-            for (int it = 0; it < kColIt; ++it) {
-                const uint32_t x = tE + uint32_t(it) * 32u * kEpiWarps;
-                if (x < uint32_t(kUnitCols)) S.nbk[x] = int32_t((31u - (x & 31u)) - (nb[it] << 8));
-            }
-            named_bar(1, 32 * kEpiWarps);
-            for (uint32_t b = 0; b < U.cb; ++b) {
-                const uint32_t blockBase = U.c0 + 128u * b;
-                const uint32_t jw = blockBase + 32u * kCPW * wg;  // first column of this warp (row side)
-                // Column side: this thread's column of the block is 32 q + lane; its rows in every
-                // tile are the warpgroup's slice 32 (kCPW wg + cc) + k, k < 32. colBest[cc] is the
-                // best column key over the slice's rows of all the unit's tiles.
-                int32_t colBest[kCPW];
-#pragma unroll
-                for (int cc = 0; cc < kCPW; ++cc) colBest[cc] = INT32_MIN;
-#pragma unroll 1
-                for (uint32_t p = 0; p < U.pt; ++p) {
-                    const uint32_t r = 128u * p + t128;
-                    const int32_t rowcP = S.rowc[r];
-                    // Trigger threshold: strictly better than this warpgroup's best (its columns
-                    // come in increasing order), and no worse than the global best.
-                    int32_t tkP = S.tk[wg][r], l2kP = S.l2k[wg][r];
-                    const uint32_t buf = acc % kAccBufs;
-                    mbar_wait(&S.accFull[buf], (acc / kAccBufs) & 1u, err, kDevTimeoutAccFull);
-                    tc_fence_after();
-                    uint32_t x[32 * kCPW], y[32 * kCPW];
-#pragma unroll
-                    for (int cc = 0; cc < kCPW; ++cc) {
-                        const uint32_t col = buf * kAccCols + 32u * (kCPW * wg + cc);
-                        tmem_ld32(tmem + laneBase + col, *reinterpret_cast<uint32_t(*)[32]>(&x[32 * cc]));
-                        tmem_ld32(tmem + laneBase + col + 128u, *reinterpret_cast<uint32_t(*)[32]>(&y[32 * cc]));
-                    }
-                    tmem_wait_ld();
-                    // The accumulators are in registers now: hand the TMEM buffer back to the MMA.
-                    tc_fence_before();  // (tcgen05.ld and its wait are warp-collective: the warp is converged)
-                    if (lane == 0) mbar_arrive(&S.accEmpty[buf]);
-                    ++acc;
-                    // ---- column side: ck = (dot << 9) + rowc of the row (ties -> smallest row)
-#pragma unroll
-                    for (int cc = 0; cc < kCPW; ++cc) {
-                        int32_t m[4] = {INT32_MIN, INT32_MIN, INT32_MIN, INT32_MIN};
-                        const int4* rc4 = reinterpret_cast<const int4*>(&S.rowc[128u * p + 32u * (kCPW * wg + cc)]);
-#pragma unroll
-                        for (int k8 = 0; k8 < 4; ++k8) {
-                            const int4 va = rc4[2 * k8], vb = rc4[2 * k8 + 1];
-                            const int32_t rcv[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
-                            int32_t ck[8];
-#pragma unroll
-                            for (int e8 = 0; e8 < 8; ++e8)
-                                ck[e8] = int32_t((y[32 * cc + 8 * k8 + e8] << 9) + uint32_t(rcv[e8]));
-#pragma unroll
-                            for (int e4 = 0; e4 < 4; ++e4) m[e4] = __vimax3_s32(m[e4], ck[e4], ck[e4 + 4]);
-                        }
-                        colBest[cc] = max(colBest[cc], max(max(m[0], m[1]), max(m[2], m[3])));
-                    }
-                    // ---- row side: row keys without the row constant, rk' = (dot << 9) + nbk;
-                    // the row key of the thresholds is rk' + rowc.
-#pragma unroll
-                    for (int cc = 0; cc < kCPW; ++cc) {
-                        const uint32_t j0 = jw + 32u * cc;
-                        int32_t m[4] = {INT32_MIN, INT32_MIN, INT32_MIN, INT32_MIN};
-                        const int4* nb4 = reinterpret_cast<const int4*>(&S.nbk[j0 - U.c0]);
-#pragma unroll
-                        for (int k8 = 0; k8 < 4; ++k8) {
-                            const int4 va = nb4[2 * k8], vb = nb4[2 * k8 + 1];
-                            const int32_t nbv[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
-                            int32_t rk[8];
-#pragma unroll
-                            for (int e8 = 0; e8 < 8; ++e8) {
-                                const int k = 32 * cc + 8 * k8 + e8;
-                                // Modular 32-bit arithmetic: the true keys always fit in int32.
-                                rk[e8] = int32_t((x[k] << 9) + uint32_t(nbv[e8]));
-                                x[k] = uint32_t(rk[e8]);
-                            }
-#pragma unroll
-                            for (int e4 = 0; e4 < 4; ++e4) m[e4] = __vimax3_s32(m[e4], rk[e4], rk[e4 + 4]);
-                        }
-                        // Chunk keys x[] and their maximum R live in a space offset by `off` from
-                        // the row-key space (off = rowc; 0 after the ragged-edge conversion).
-                        int32_t R = max(max(m[0], m[1]), max(m[2], m[3]));
-                        int32_t off = rowcP;
-                        // Columns past nbDescB only occur in a task's last block: drop them there.
-                        if (j0 + 32u > T.nB) {
-                            R = INT32_MIN;
-                            off = 0;
-#pragma unroll
-                            for (int k = 0; k < 32; ++k) {
-                                x[32 * cc + k] = (j0 + k >= T.nB) ? uint32_t(INT32_MIN) : x[32 * cc + k] + uint32_t(rowcP);
-                                R = max(R, int32_t(x[32 * cc + k]));
-                            }
-                        }
-                        const int32_t rmax = int32_t(uint32_t(R) + uint32_t(off));
-                        if (__any_sync(0xffffffffu, rmax >= tkP)) {
-                            // Second key of the chunk: keys within a chunk are distinct, so
-                            // min over k of (R - 1 - key) (unsigned) skips exactly the maximum.
-                            uint32_t mn = 0xFFFFFFFFu;
-#pragma unroll
-                            for (int k = 0; k < 32; ++k) mn = min(mn, uint32_t(R) - 1u - x[32 * cc + k]);
-                            const int32_t s2 = int32_t(uint32_t(R) - 1u - mn + uint32_t(off));
-                            if (rmax >= tkP) {
-                                const uint32_t c = uint32_t(rowcP) & 255u;
-                                // the previous own best (key of distance d1: tk - 256) becomes a second
-                                if (S.l1j[wg][r] != 0xFFFFu) l2kP = max(l2kP, int32_t(uint32_t(tkP) - 256u));
-                                l2kP = max(l2kP, s2);
-                                S.l1j[wg][r] = uint16_t((j0 - U.c0) + 31u - ((uint32_t(rmax) - c) & 255u));
-                                tkP = int32_t((uint32_t(rmax) - ((uint32_t(rmax) - c) & 255u)) + 256u);
-                                S.tk[wg][r] = tkP;
-                            } else {
-                                l2kP = max(l2kP, rmax);
-                            }
+        };
+        for (uint32_t u = blockIdx.x; u < P.totalUnits; u += gridDim.x, ++k) {
+            const uint32_t slot = k & 1u;
+            mbar_wait(&S.aReady[slot], (k >> 1) & 1u, err, kDevTimeoutAccFull);
+            const UnitInfo& I = S.info[slot];
+            // (read from shared memory where it is used: registers are short here)
+            // residuals of the rows (transposes), if the row half has any
+            const bool resA = (S.flagA[slot][inner >> 6] | S.flagA[slot][(inner >> 6) + 1]) != 0u;
+            // keys: (value - centre) << 8 | code, the code falling with the chunk's position
+            uint32_t baseR = 255u - (I.cB << 8);
+            const uint32_t baseC = 255u - (I.cA << 8);
+            int32_t l1 = INT_MIN, l2 = INT_MIN;  // the row's best chunk and (kSecond) the next
+            uint32_t thrA = ~0u;  // row distances from here on change nothing
+            for (uint32_t c = 0; c < I.cols; c += kBlockCols, baseR -= 8u) {
+                mbar_wait(&S.bReady[stage], bPhase, err, kDevTimeoutAccFull);
+                // A column's value below thr cannot change its result, which only falls (a tie can:
+                // the lower index wins). Loaded here, used after the tile.
+                int32_t thr = INT_MAX;
+                if (mine < I.cols - c) {
+                    const uint32_t d = __ldcg(reinterpret_cast<const uint32_t*>(&I.bestB[I.c0 + c + mine]) + 1);
+                    thr = max(int32_t(S.nrmB[stage][mine] - min(d, 1u << 24)), kNoValue + 1);
+                }
+                if (I.cols - c <= kBlockCols && mine < I.rows) {  // last block: the row's results by now
+                    thrA = __ldcg(reinterpret_cast<const uint32_t*>(&I.bestA[I.r0 + mine]) + 1);
+                    thrA = min(thrA, ~1u) + 1u;
+                    if (kSecond) thrA = max(thrA, __ldcg(&I.secondA[I.r0 + mine]));
+                }
+                if (outer < I.rows) {
+                    const bool any = (S.flagB[stage][inner >> 6] | S.flagB[stage][(inner >> 6) + 1]) != 0u;
+                    chunks(any ? &S.resB[stage][inner] : nullptr, baseR, [&](int32_t k0, int32_t k1) {
+                        if (kSecond) {
+                            const int32_t hi = max(k0, k1);
+                            l2 = __vimax3_s32(l2, min(k0, k1), min(l1, hi));
+                            l1 = max(l1, hi);
                         } else {
-                            l2kP = max(l2kP, rmax);
+                            l1 = __vimax3_s32(l1, k0, k1);
                         }
-                    }
-                    S.l2k[wg][r] = l2kP;
+                    });
                 }
-                // ---- column publish: one global atomic per (column, row slice); no cross-warp
-                // step. Key = (|b|^2 - d) * 256 + code, code = (7 - p) << 5 | (31 - k).
-                const uint32_t jb = 32u * q + lane;  // column within the block
-                const uint32_t j = blockBase + jb;
-                if (j < T.nB) {
-                    const uint32_t xj = j - U.c0;  // |b_j|^2 from the staged row-key addend
-                    const uint32_t nbj = ((31u - (xj & 31u)) - uint32_t(S.nbk[xj])) >> 8;
-#pragma unroll
-                    for (int cc = 0; cc < kCPW; ++cc) {
-                        const uint32_t code = uint32_t(colBest[cc]) & 255u;
-                        const uint32_t rr = 128u * (7u - (code >> 5)) + 32u * (kCPW * wg + cc) + (31u - (code & 31u));
-                        const uint32_t i = U.r0 + rr;
-                        if (i < T.nA) {
-                            const uint32_t d = nbj - uint32_t(colBest[cc] >> 8);
-                            red_min_u64(&T.bestB[j], (static_cast<unsigned long long>(d) << 32) | i);
-                        }
+                if (outer < I.cols - c) {
+                    int32_t best = INT_MIN;
+                    chunks(resA ? &S.resA[slot][inner] : nullptr, baseC, [&](int32_t k0, int32_t k1) {
+                        best = __vimax3_s32(best, k0, k1);
+                    });
+                    if ((best >> 8) >= thr) {
+                        const uint32_t d = S.nrmB[stage][mine] - uint32_t(best >> 8);
+                        const uint32_t i = I.r0 + inner + kChunk * (255u - (uint32_t(best) & 255u));
+                        red_min_u64(&I.bestB[I.c0 + c + mine], (static_cast<unsigned long long>(d) << 32) | i);
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&S.bEpi[stage]);
+                if (++stage == uint32_t(kBStages)) { stage = 0; bPhase ^= 1u; }
+            }
+            // ---- the unit's rows: best chunk of this column half, merged by atomics with the others
+            if (mine < I.rows && (l1 >> 8) != kNoValue) {
+                const uint32_t na = S.nrmA[slot][mine];
+                const uint32_t d1 = na - uint32_t(l1 >> 8);
+                const uint32_t idx = 255u - (uint32_t(l1) & 255u);
+                const unsigned long long key = (static_cast<unsigned long long>(d1) << 32) |
+                                               (I.c0 + kBlockCols * (idx >> 3) + inner + kChunk * (idx & 7u));
+                if (d1 < thrA) {
+                    if (kSecond) {
+                        const unsigned long long old = atomicMin(&I.bestA[I.r0 + mine], key);
+                        uint32_t s = max(uint32_t(old >> 32), d1);
+                        if ((l2 >> 8) != kNoValue) s = min(s, na - uint32_t(l2 >> 8));
+                        red_min_u32(&I.secondA[I.r0 + mine], s);
+                    } else {
+                        red_min_u64(&I.bestA[I.r0 + mine], key);
                     }
                 }
             }
-            // ---- unit end: merge the warpgroups' row states (exact two-slot merge) and publish
-            // each row once: old = atomicMin(best, b); second = min(second, max(old, b), s).
-            named_bar(1, 32 * kEpiWarps);
-#pragma unroll 1
-            for (uint32_t r = tE; r < 128u * U.pt; r += 32u * kEpiWarps) {
-                const uint32_t i = U.r0 + r;
-                if (i >= T.nA) continue;
-                const uint32_t c = uint32_t(S.rowc[r]) & 255u;
-                unsigned long long bst = ~0ull;
-                uint32_t sec = ~0u;
-#pragma unroll
-                for (int w = 0; w < kWG; ++w) {
-                    const int32_t k2 = S.l2k[w][r];
-                    if (S.l1j[w][r] != 0xFFFFu) {  // tk = -(d1 - 1) * 256 + c
-                        const uint32_t d1 = 1u - uint32_t(int32_t(uint32_t(S.tk[w][r]) - c) >> 8);
-                        const unsigned long long key =
-                            (static_cast<unsigned long long>(d1) << 32) | (U.c0 + uint32_t(S.l1j[w][r]));
-                        if (key < bst) {
-                            sec = min(sec, uint32_t(bst >> 32));
-                            bst = key;
-                        } else {
-                            sec = min(sec, d1);
-                        }
-                    }
-                    if (k2 != INT32_MIN) sec = min(sec, 0u - uint32_t(int32_t(uint32_t(k2) - c) >> 8));
-                }
-                if (bst != ~0ull) {
-                    const unsigned long long old = atomicMin(&T.bestA[i], bst);
-                    red_min_u32(&T.secondA[i], max(uint32_t(old >> 32), uint32_t(bst >> 32)));
-                }
-                if (sec != ~0u) red_min_u32(&T.secondA[i], sec);
-            }
-            named_bar(1, 32 * kEpiWarps);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&S.aEpi[slot]);
         }
     }
 
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, 512);
+    __syncwarp();
+
+    if (!P.fused) return;
+    // ---- every unit of the launch is published: indexes inside the winning chunks, then the flags,
+    // as phases of one cooperative launch (all CTAs are resident, and every wait above ends)
+    const cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+    grid.sync();
+    const uint32_t warps = gridDim.x * (kThreads / 32u), w0 = blockIdx.x * (kThreads / 32u) + warp;
+    resolve_phase(P, w0, warps, lane);
+    if (kSecond && P.totalRowGroups > 0) {
+        grid.sync();
+        flags_phase(P, w0, warps, lane);
+    }
+}
+
+// The same two phases as launches of their own.
+__global__ void __launch_bounds__(256) bf_resolve_kernel(const __grid_constant__ Params P) {
+    resolve_phase(P, blockIdx.x * 8u + (threadIdx.x >> 5), gridDim.x * 8u, threadIdx.x & 31u);
+}
+__global__ void __launch_bounds__(256) bf_flags_kernel(const __grid_constant__ Params P) {
+    flags_phase(P, blockIdx.x * 8u + (threadIdx.x >> 5), gridDim.x * 8u, threadIdx.x & 31u);
 }
 
 // Initialise results: bestA/bestB = {~0u, ~0u}, secondA = ~0u.
-struct InitParams {
-    unsigned long long* bestA[kMaxTasksPerLaunch];
-    unsigned long long* bestB[kMaxTasksPerLaunch];
-    uint32_t* secondA[kMaxTasksPerLaunch];
-    uint32_t nA[kMaxTasksPerLaunch], nB[kMaxTasksPerLaunch];
-};
 __global__ void bf_init_kernel(const __grid_constant__ InitParams P) {
     const uint32_t t = blockIdx.y;
     const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x < P.nA[t]) {
         P.bestA[t][x] = ~0ull;
-        P.secondA[t][x] = ~0u;
+        if (P.secondA[t]) P.secondA[t][x] = ~0u;
     }
     if (x < P.nB[t]) P.bestB[t][x] = ~0ull;
-}
-
-// Flags: bit0 ratio test, bit1 cross-check.
-struct FlagParams {
-    const unsigned long long* bestA[kMaxTasksPerLaunch];
-    const unsigned long long* bestB[kMaxTasksPerLaunch];
-    const uint32_t* secondA[kMaxTasksPerLaunch];
-    uint32_t* flagsA[kMaxTasksPerLaunch];
-    uint32_t nA[kMaxTasksPerLaunch], nB[kMaxTasksPerLaunch];
-    uint32_t ratioNum, ratioDen;
-};
-__global__ void bf_flags_kernel(const __grid_constant__ FlagParams P) {
-    const uint32_t t = blockIdx.y;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.nA[t]) return;
-    const unsigned long long bm = P.bestA[t][i];
-    const uint32_t j = uint32_t(bm & 0xFFFFFFFFu);
-    const uint32_t d = uint32_t(bm >> 32);
-    uint32_t f = 0;
-    if (j != ~0u) {
-        const uint64_t lhs = uint64_t(P.ratioDen) * d;
-        const uint64_t rhs = uint64_t(P.ratioNum) * P.secondA[t][i];
-        if (lhs < rhs) f |= 1u;
-        if (j < P.nB[t] && uint32_t(P.bestB[t][j] & 0xFFFFFFFFu) == i) f |= 2u;
-    }
-    P.flagsA[t][i] = f;
 }
 
 // ---------------------------------------------------------------- squared norms
@@ -554,77 +709,120 @@ __global__ void sqr_norm_kernel(uint32_t* __restrict__ out, const uint4* __restr
     if (i < n && part == 0) out[i] = acc;
 }
 
-template <int kWG>
-static size_t smem_bytes() { return sizeof(Smem<kWG>) + 1024; }
-
-// Unit shape: as many A rows per unit as possible (fewer column atomics), then columns, keeping
-// at least ~2 units per SM when the problem allows.
-static void choose_shape(const std::vector<std::pair<uint32_t, uint32_t>>& sizes, int nsm, uint32_t& rowTiles,
-                         uint32_t& colBlocks) {
-    auto count = [&](uint32_t rt, uint32_t cbk) {
-        uint64_t total = 0;
+// 256-column blocks per unit. A CTA spends about 1.4 us of tensor time on a block (four products)
+// and about 0.9 us more on a unit when the next unit's rows are not ready in time (units of fewer
+// than four blocks) or 0.15 us when they are; the launch lasts as long as the CTA with the most
+// units. The shape with the shortest estimate is taken, the longer unit on a tie (fewer row publishes).
+static uint32_t choose_unit_blocks(const std::vector<std::pair<uint32_t, uint32_t>>& sizes, int nsm) {
+    uint32_t pick = 1;
+    double best = 0;
+    for (uint32_t ub : {16u, 8u, 4u, 2u, 1u}) {
+        uint64_t units = 0, blocks = 0;
         for (auto& s : sizes) {
-            const uint64_t rb = (s.first + 128u * rt - 1) / (128u * rt);
-            const uint64_t cr = (s.second + 128u * cbk - 1) / (128u * cbk);
-            total += rb * cr;
+            const uint64_t rb = (s.first + kUnitRows - 1) / kUnitRows;
+            const uint64_t nb = (s.second + kBlockCols - 1) / kBlockCols;
+            units += rb * ((nb + ub - 1) / ub);
+            blocks += rb * nb;
         }
-        return total;
-    };
-    const uint64_t want = uint64_t(nsm) * 4;
-    for (uint32_t rt : {8u, 4u, 2u}) {
-        for (uint32_t cbk : {8u, 4u, 2u, 1u}) {
-            if (count(rt, cbk) >= want) {
-                rowTiles = rt;
-                colBlocks = cbk;
-                return;
-            }
+        if (units == 0) return 1;
+        const uint64_t waves = (units + uint64_t(nsm) - 1) / uint64_t(nsm);
+        const double perUnit = 1.4 * double(blocks) / double(units) + (ub >= 4 ? 0.15 : 0.9);
+        const double est = double(waves) * perUnit;
+        if (best == 0 || est < 0.98 * best) {
+            best = est;
+            pick = ub;
         }
     }
-    rowTiles = 2;
-    colBlocks = 1;
+    return pick;
 }
 
-// Epilogue warpgroups (4 by default, or 2); RSFM_BF_EPILOGUE_GROUPS overrides it for tuning runs.
-static int epilogue_groups() {
-    static int g = [] {
-        const char* e = getenv("RSFM_BF_EPILOGUE_GROUPS");
-        return (e && atoi(e) == 2) ? 2 : 4;
-    }();
-    return g;
-}
-
-template <int kWG>
+template <bool kSecond>
 static int ensure_attr() {
-    return set_max_dynamic_smem(reinterpret_cast<const void*>(bf_match_kernel<kWG>), smem_bytes<kWG>());
+    return set_max_dynamic_smem(reinterpret_cast<const void*>(bf_match_kernel<kSecond>), sizeof(Smem) + 1024);
 }
 
-template <int kWG>
-static int launch_main(const Params& P, uint32_t grid, cudaStream_t stream) {
-    const int st = ensure_attr<kWG>();
+// Up to eight blocks per SM a call is bound by its host time (2 us a launch), so matching, index
+// resolution and flags share one launch; beyond, the grid-wide barriers between them cost more than
+// launches (897 x 1013: 38 against 44 us a call; 32768 x 32768: 274 against 251 us).
+static bool fuse_phases(const Params& P, int nsm) {
+    return uint64_t(P.totalUnits) * P.unitBlocks <= uint64_t(nsm) * 8;
+}
+
+// The matcher and what follows it.
+template <bool kSecond>
+static int launch_match(const Params& P, int nsm, cudaStream_t stream) {
+    const int st = ensure_attr<kSecond>();
     if (st != RSFM_OK) return st;
-    bf_match_kernel<kWG><<<grid, Cfg<kWG>::kThreads, smem_bytes<kWG>(), stream>>>(P);
-    RSFM_CUDA_TRY(cudaGetLastError());
+    void* tok = nullptr;
+    const bool prof = profile_begin(stream, &tok);
+    if (P.fused) {
+        // a CTA per unit, or enough for the results of a few units with many columns
+        const uint32_t want = std::max(P.totalUnits, std::max(P.totalGroups, P.totalRowGroups) / (kThreads / 32) + 1);
+        void* args[] = {const_cast<Params*>(&P)};
+        RSFM_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(bf_match_kernel<kSecond>),
+                                                  dim3(std::min<uint32_t>(want, uint32_t(nsm))), dim3(kThreads), args,
+                                                  sizeof(Smem) + 1024, stream));
+    } else if (P.totalUnits > 0) {
+        bf_match_kernel<kSecond><<<std::min<uint32_t>(P.totalUnits, uint32_t(nsm)), kThreads, sizeof(Smem) + 1024, stream>>>(P);
+        RSFM_CUDA_TRY(cudaGetLastError());
+    }
+    if (prof) profile_end(stream, tok);
+    launch_count_add(1);
+    if (P.fused) return RSFM_OK;
+    if (P.totalGroups > 0) {
+        bf_resolve_kernel<<<std::min<uint32_t>((P.totalGroups + 7) / 8, uint32_t(nsm) * 64u), 256, 0, stream>>>(P);
+        RSFM_CUDA_TRY(cudaGetLastError());
+        launch_count_add(1);
+    }
+    if (P.totalRowGroups > 0) {
+        bf_flags_kernel<<<std::min<uint32_t>((P.totalRowGroups + 7) / 8, uint32_t(nsm) * 64u), 256, 0, stream>>>(P);
+        RSFM_CUDA_TRY(cudaGetLastError());
+        launch_count_add(1);
+    }
+    return RSFM_OK;
+}
+
+// Fills a task's device description and counts it into P's totals. Empty sides get no units.
+static int fill_task(TaskDev* T, const rsfm_sift_bf_task& in, uint32_t* second, uint32_t* flags, Params* P) {
+    T->nA = in.nbDescA;
+    T->nB = in.nbDescB;
+    T->descA = static_cast<const uint4*>(in.descA);
+    T->descB = static_cast<const uint4*>(in.descB);
+    T->sqrA = in.sqrNormDescA;
+    T->sqrB = in.sqrNormDescB;
+    T->bestA = reinterpret_cast<unsigned long long*>(in.bestMatchA);
+    T->bestB = reinterpret_cast<unsigned long long*>(in.bestMatchB);
+    T->secondA = second;
+    T->flagsA = flags;
+    T->unitBegin = P->totalUnits;
+    T->groupBegin = P->totalGroups;
+    T->rowGroupBegin = P->totalRowGroups;
+    T->rowBlocks = 1;
+    if (flags) P->totalRowGroups += (T->nA + 31) / 32;
+    if (T->nA == 0 || T->nB == 0) return RSFM_OK;
+    int st = encode_desc_tmap(&T->tmA, in.descA, T->nA, kUnitRows);
+    if (st == RSFM_OK) st = encode_desc_tmap(&T->tmB, in.descB, T->nB, kBlockCols);
+    if (st != RSFM_OK) return st;
+    T->rowBlocks = (T->nA + kUnitRows - 1) / kUnitRows;
+    const uint32_t unitCols = kBlockCols * P->unitBlocks;
+    P->totalUnits += T->rowBlocks * ((T->nB + unitCols - 1) / unitCols);
+    P->totalGroups += uint32_t((uint64_t(T->nA) + T->nB + 3) / 4);
     return RSFM_OK;
 }
 
 int launch_chunk(const rsfm_sift_bf_task* tasks, size_t n, uint32_t* const* second, uint32_t* const* flags,
-                 uint32_t ratioNum, uint32_t ratioDen, cudaStream_t stream) {
+                 uint32_t ratioNum, uint32_t ratioDen, cudaStream_t stream, bool initialised) {
     const int nsm = sm_count();
     if (nsm <= 0) return RSFM_ERR_CUDA;
 
-    InitParams ip{};
+    const InitParams ip = init_params(tasks, n, second);
     uint32_t maxN = 0;
     std::vector<std::pair<uint32_t, uint32_t>> sizes;
     for (size_t t = 0; t < n; ++t) {
-        ip.bestA[t] = reinterpret_cast<unsigned long long*>(tasks[t].bestMatchA);
-        ip.bestB[t] = reinterpret_cast<unsigned long long*>(tasks[t].bestMatchB);
-        ip.secondA[t] = second[t];
-        ip.nA[t] = tasks[t].nbDescA;
-        ip.nB[t] = tasks[t].nbDescB;
         maxN = std::max(maxN, std::max(tasks[t].nbDescA, tasks[t].nbDescB));
         sizes.emplace_back(tasks[t].nbDescA, tasks[t].nbDescB);
     }
-    if (maxN > 0) {
+    if (maxN > 0 && !initialised) {
         dim3 g((maxN + 255) / 256, uint32_t(n));
         bf_init_kernel<<<g, 256, 0, stream>>>(ip);
         RSFM_CUDA_TRY(cudaGetLastError());
@@ -633,72 +831,27 @@ int launch_chunk(const rsfm_sift_bf_task* tasks, size_t n, uint32_t* const* seco
 
     Params P;
     memset(&P, 0, sizeof(P));
-    choose_shape(sizes, nsm, P.rowTiles, P.colBlocks);
-    uint32_t units = 0;
+    P.unitBlocks = choose_unit_blocks(sizes, nsm);
+    P.ratioNum = ratioNum;
+    P.ratioDen = ratioDen;
     for (size_t t = 0; t < n; ++t) {
-        TaskDev& T = P.tasks[t];
-        const rsfm_sift_bf_task& in = tasks[t];
-        T.nA = in.nbDescA;
-        T.nB = in.nbDescB;
-        T.sqrA = in.sqrNormDescA;
-        T.sqrB = in.sqrNormDescB;
-        T.bestA = reinterpret_cast<unsigned long long*>(in.bestMatchA);
-        T.bestB = reinterpret_cast<unsigned long long*>(in.bestMatchB);
-        T.secondA = second[t];
-        T.unitBegin = units;
-        if (T.nA == 0 || T.nB == 0) {
-            T.rowBlocks = 1;
-            T.colRanges = 0;
-            continue;
-        }
-        int st = encode_desc_tmap(&T.tmA, in.descA, T.nA, 128);
+        const int st = fill_task(&P.tasks[t], tasks[t], ip.secondA[t], flags ? flags[t] : nullptr, &P);
         if (st != RSFM_OK) return st;
-        st = encode_desc_tmap(&T.tmB, in.descB, T.nB, 128);
-        if (st != RSFM_OK) return st;
-        T.rowBlocks = (T.nA + 128u * P.rowTiles - 1) / (128u * P.rowTiles);
-        T.colRanges = (T.nB + 128u * P.colBlocks - 1) / (128u * P.colBlocks);
-        units += T.rowBlocks * T.colRanges;
     }
     P.nTasks = uint32_t(n);
-    P.totalUnits = units;
     P.err = device_error_word();
     if (!P.err) return RSFM_ERR_CUDA;
-    if (units > 0) {
-        const uint32_t grid = std::min<uint32_t>(units, uint32_t(nsm));
-        void* tok = nullptr;
-        const bool prof = profile_begin(stream, &tok);
-        const int st = epilogue_groups() == 4 ? launch_main<4>(P, grid, stream) : launch_main<2>(P, grid, stream);
+    if (P.totalUnits > 0 || P.totalRowGroups > 0) {
+        P.fused = fuse_phases(P, nsm) ? 1u : 0u;
+        const int st = second ? launch_match<true>(P, nsm, stream) : launch_match<false>(P, nsm, stream);
         if (st != RSFM_OK) return st;
-        if (prof) profile_end(stream, tok);
-        launch_count_add(1);
-    }
-    if (flags) {
-        FlagParams fp{};
-        uint32_t maxA = 0;
-        for (size_t t = 0; t < n; ++t) {
-            fp.bestA[t] = ip.bestA[t];
-            fp.bestB[t] = ip.bestB[t];
-            fp.secondA[t] = second[t];
-            fp.flagsA[t] = flags[t];
-            fp.nA[t] = tasks[t].nbDescA;
-            fp.nB[t] = tasks[t].nbDescB;
-            maxA = std::max(maxA, tasks[t].nbDescA);
-        }
-        fp.ratioNum = ratioNum;
-        fp.ratioDen = ratioDen;
-        if (maxA > 0) {
-            dim3 g((maxA + 255) / 256, uint32_t(n));
-            bf_flags_kernel<<<g, 256, 0, stream>>>(fp);
-            RSFM_CUDA_TRY(cudaGetLastError());
-            launch_count_add(1);
-        }
     }
     return RSFM_OK;
 }
 
 // ---------------------------------------------------------------- batched plans
 // A plan holds the tasks of a whole batch (any count) in device memory, so the matcher runs as
-// one persistent launch over all (task, row block, column range) units; init, match and flags
+// one persistent launch over all (task, row block, column range) units; init and match
 // are captured once in a CUDA graph and replayed.
 __global__ void plan_init_kernel(const TaskDev* __restrict__ tasks) {
     const TaskDev& T = tasks[blockIdx.y];
@@ -710,28 +863,15 @@ __global__ void plan_init_kernel(const TaskDev* __restrict__ tasks) {
         if (x < T.nB) T.bestB[x] = ~0ull;
     }
 }
-__global__ void plan_flags_kernel(const TaskDev* __restrict__ tasks, uint32_t ratioNum, uint32_t ratioDen) {
-    const TaskDev& T = tasks[blockIdx.y];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < T.nA; i += gridDim.x * blockDim.x) {
-        const unsigned long long bm = T.bestA[i];
-        const uint32_t j = uint32_t(bm & 0xFFFFFFFFu), d = uint32_t(bm >> 32);
-        uint32_t f = 0;
-        if (j != ~0u) {
-            if (uint64_t(ratioDen) * d < uint64_t(ratioNum) * T.secondA[i]) f |= 1u;
-            if (j < T.nB && uint32_t(T.bestB[j] & 0xFFFFFFFFu) == i) f |= 2u;
-        }
-        T.flagsA[i] = f;
-    }
-}
-
 }  // namespace bf
 }  // namespace rsfm_b200
 
 struct rsfm_bf_plan {
     rsfm_b200::bf::TaskDev* dTasks = nullptr;
     rsfm_b200::bf::Params P;
-    uint32_t grid = 0, nTasks = 0, ratioNum = 64, ratioDen = 100, groups = 2;
+    uint32_t nTasks = 0;
     uint32_t blocksX = 1;
+    int nsm = 0;
     cudaStream_t capture = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -745,15 +885,7 @@ static int plan_enqueue(rsfm_bf_plan* pl, cudaStream_t s) {
     launch_count_add(1);
     plan_init_kernel<<<dim3(pl->blocksX, pl->nTasks), 256, 0, s>>>(pl->dTasks);
     RSFM_CUDA_TRY(cudaGetLastError());
-    if (pl->P.totalUnits > 0) {
-        const int st = pl->groups == 4 ? launch_main<4>(pl->P, pl->grid, s) : launch_main<2>(pl->P, pl->grid, s);
-        if (st != RSFM_OK) return st;
-        launch_count_add(1);
-    }
-    plan_flags_kernel<<<dim3(pl->blocksX, pl->nTasks), 256, 0, s>>>(pl->dTasks, pl->ratioNum, pl->ratioDen);
-    RSFM_CUDA_TRY(cudaGetLastError());
-    launch_count_add(1);
-    return RSFM_OK;
+    return launch_match<true>(pl->P, pl->nsm, s);
 }
 
 int validate(const rsfm_sift_bf_task* tasks, size_t n) {
@@ -810,32 +942,12 @@ extern "C" int rsfm_bf_match(const rsfm_sift_bf_task* tasks, size_t nbTasks, cud
     int st = bf::validate(tasks, nbTasks);
     if (st != RSFM_OK) return st;
     if (nbTasks == 0) return RSFM_OK;
-    // The second-best distances drive the row thresholds; the reference API has no output for
-    // them, so they live in stream-ordered scratch here.
-    size_t total = 0;
-    for (size_t t = 0; t < nbTasks; ++t) total += tasks[t].nbDescA;
-    uint32_t* scratch = nullptr;
-    if (total > 0) {
-        cudaMemPool_t pool = nullptr;
-        const int ps = scratch_pool(&pool);
-        if (ps != RSFM_OK) return ps;
-        RSFM_CUDA_TRY(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&scratch), total * 4, pool, stream));
-    }
-    std::vector<uint32_t*> second(nbTasks);
-    size_t off = 0;
-    for (size_t t = 0; t < nbTasks; ++t) {
-        second[t] = scratch ? scratch + off : nullptr;
-        off += tasks[t].nbDescA;
-    }
-    for (size_t i = 0; i < nbTasks && st == RSFM_OK; i += bf::kMaxTasksPerLaunch) {
+    for (size_t i = 0; i < nbTasks; i += bf::kMaxTasksPerLaunch) {
         const size_t n = std::min<size_t>(bf::kMaxTasksPerLaunch, nbTasks - i);
-        st = bf::launch_chunk(tasks + i, n, second.data() + i, nullptr, 0, 1, stream);
+        st = bf::launch_chunk(tasks + i, n, nullptr, nullptr, 0, 1, stream);
+        if (st != RSFM_OK) return st;
     }
-    if (scratch) {
-        cudaError_t e = cudaFreeAsync(scratch, stream);
-        if (st == RSFM_OK && e != cudaSuccess) st = RSFM_ERR_CUDA;
-    }
-    return st;
+    return RSFM_OK;
 }
 
 extern "C" int rsfm_bf_plan_create(const rsfm_sift_bf_task* tasks, size_t nbTasks, uint32_t* const* secondDistA,
@@ -857,12 +969,14 @@ extern "C" int rsfm_bf_plan_create(const rsfm_sift_bf_task* tasks, size_t nbTask
         sizes.emplace_back(tasks[t].nbDescA, tasks[t].nbDescB);
         maxN = std::max(maxN, std::max(tasks[t].nbDescA, tasks[t].nbDescB));
     }
-    uint32_t rt = 0, cb = 0;
-    bf::choose_shape(sizes, nsm, rt, cb);
-    if (opts && opts->rowTiles) rt = std::min<uint32_t>(opts->rowTiles, bf::kMaxRowTiles);
-    if (opts && opts->colBlocks) cb = std::min<uint32_t>(opts->colBlocks, bf::kMaxColBlocks);
-    pl->groups = (opts && opts->epilogueGroups == 4) ? 4u : (opts && opts->epilogueGroups == 2) ? 2u
-                                                                                                : uint32_t(bf::epilogue_groups());
+    // The options give a unit as rowTiles x colBlocks tiles of 128 x 128; units here are 256 rows
+    // high, so the same area is taken as 256-column blocks.
+    uint32_t ub = bf::choose_unit_blocks(sizes, nsm);
+    if (opts && (opts->rowTiles || opts->colBlocks)) {
+        const uint32_t rt = opts->rowTiles ? std::min<uint32_t>(opts->rowTiles, 8) : 8;
+        const uint32_t cb = opts->colBlocks ? std::min<uint32_t>(opts->colBlocks, 8) : 8;
+        ub = std::max<uint32_t>(1, rt * cb / 4);
+    }
     // Unit order: pairs in the given order, or largest pairs first (their units are spread over
     // every CTA before the small pairs fill the tail).
     std::vector<size_t> order(nbTasks);
@@ -872,31 +986,14 @@ extern "C" int rsfm_bf_plan_create(const rsfm_sift_bf_task* tasks, size_t nbTask
             return uint64_t(tasks[x].nbDescA) * tasks[x].nbDescB > uint64_t(tasks[y].nbDescA) * tasks[y].nbDescB;
         });
     std::vector<bf::TaskDev> host(nbTasks);
-    uint32_t units = 0;
+    pl->P.unitBlocks = ub;
     for (size_t o = 0; o < nbTasks; ++o) {
         const size_t t = order[o];
         bf::TaskDev& T = host[o];
         memset(&T, 0, sizeof(T));
-        const rsfm_sift_bf_task& in = tasks[t];
-        T.nA = in.nbDescA;
-        T.nB = in.nbDescB;
-        T.sqrA = in.sqrNormDescA;
-        T.sqrB = in.sqrNormDescB;
-        T.bestA = reinterpret_cast<unsigned long long*>(in.bestMatchA);
-        T.bestB = reinterpret_cast<unsigned long long*>(in.bestMatchB);
-        T.secondA = secondDistA[t];
-        T.flagsA = flagsA[t];
-        T.unitBegin = units;
-        T.rowBlocks = 1;
-        if (T.nA && T.nB) {
-            if ((st = encode_desc_tmap(&T.tmA, in.descA, T.nA, 128)) != RSFM_OK ||
-                (st = encode_desc_tmap(&T.tmB, in.descB, T.nB, 128)) != RSFM_OK) {
-                delete pl;
-                return st;
-            }
-            T.rowBlocks = (T.nA + 128u * rt - 1) / (128u * rt);
-            T.colRanges = (T.nB + 128u * cb - 1) / (128u * cb);
-            units += T.rowBlocks * T.colRanges;
+        if ((st = bf::fill_task(&T, tasks[t], secondDistA[t], flagsA[t], &pl->P)) != RSFM_OK) {
+            delete pl;
+            return st;
         }
     }
     if (cudaMalloc(reinterpret_cast<void**>(&pl->dTasks), sizeof(bf::TaskDev) * nbTasks) != cudaSuccess ||
@@ -907,18 +1004,15 @@ extern "C" int rsfm_bf_plan_create(const rsfm_sift_bf_task* tasks, size_t nbTask
     pl->nTasks = uint32_t(nbTasks);
     pl->P.gtasks = pl->dTasks;
     pl->P.nTasks = uint32_t(nbTasks);
-    pl->P.totalUnits = units;
-    pl->P.rowTiles = rt;
-    pl->P.colBlocks = cb;
+    pl->P.ratioNum = ratioNum;
+    pl->P.ratioDen = ratioDen;
     pl->P.err = device_error_word();
-    pl->grid = std::min<uint32_t>(units, uint32_t(nsm));
-    pl->ratioNum = ratioNum;
-    pl->ratioDen = ratioDen;
+    pl->nsm = nsm;
     pl->blocksX = std::min<uint32_t>((maxN + 255) / 256, 64);
     const bool useGraph = !opts || opts->useGraph;
     if (useGraph) {
-        // Set kernel attributes outside the capture, then record the three launches once.
-        st = pl->groups == 4 ? bf::ensure_attr<4>() : bf::ensure_attr<2>();
+        // Set kernel attributes outside the capture, then record the launches once.
+        st = bf::ensure_attr<true>();
         if (st != RSFM_OK) {
             rsfm_bf_plan_destroy(pl);
             return st;
@@ -945,16 +1039,16 @@ extern "C" int rsfm_bf_plan_create(const rsfm_sift_bf_task* tasks, size_t nbTask
 extern "C" int rsfm_bf_plan_launch(rsfm_bf_plan* plan, cudaStream_t stream) {
     launch_count_reset();
     if (!plan) return RSFM_ERR_INVALID_ARG;
-    void* tok = nullptr;
-    const bool prof = profile_begin(stream, &tok);
     if (plan->exec) {
+        void* tok = nullptr;
+        const bool prof = profile_begin(stream, &tok);
         RSFM_CUDA_TRY(cudaGraphLaunch(plan->exec, stream));
-        launch_count_add(plan->P.totalUnits > 0 ? 3 : 2);
+        if (prof) profile_end(stream, tok);
+        launch_count_add(plan->P.totalUnits > 0 ? 4 : 2);
     } else {
         const int st = bf::plan_enqueue(plan, stream);
         if (st != RSFM_OK) return st;
     }
-    if (prof) profile_end(stream, tok);
     return RSFM_OK;
 }
 

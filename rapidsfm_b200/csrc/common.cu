@@ -1,6 +1,7 @@
 // Host helpers: tensor-map encoding, device error word, status strings, launch accounting.
 #include "common.h"
 
+#include <atomic>
 #include <mutex>
 #include <set>
 #include <utility>
@@ -22,9 +23,18 @@ void launch_count_add(uint32_t n) { t_launches += n; }
 // One word per device, written by kernels when a bounded wait gives up.
 __device__ uint32_t g_device_error = 0;
 
+// Per-device facts that every call needs: looked up once (a small call is bound by its host time).
+constexpr int kMaxDevices = 64;
+
 uint32_t* device_error_word() {
+    static std::atomic<uint32_t*> words[kMaxDevices];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+    if (dev >= 0 && dev < kMaxDevices)
+        if (uint32_t* w = words[dev].load(std::memory_order_acquire)) return w;
     void* p = nullptr;
     if (cudaGetSymbolAddress(&p, g_device_error) != cudaSuccess) return nullptr;
+    if (dev >= 0 && dev < kMaxDevices) words[dev].store(static_cast<uint32_t*>(p), std::memory_order_release);
     return static_cast<uint32_t*>(p);
 }
 
@@ -113,9 +123,12 @@ int scratch_pool(cudaMemPool_t* out) {
 }
 
 int sm_count() {
+    static std::atomic<int> counts[kMaxDevices];
     int dev = 0, n = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (dev >= 0 && dev < kMaxDevices && (n = counts[dev].load(std::memory_order_relaxed)) > 0) return n;
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    if (dev >= 0 && dev < kMaxDevices) counts[dev].store(n, std::memory_order_relaxed);
     return n;
 }
 

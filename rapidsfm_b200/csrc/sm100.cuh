@@ -11,8 +11,8 @@
 namespace rsfm_b200 {
 namespace sm100 {
 
-// A poll suspends for up to 1 us in hardware (try_wait suspend-time hint); the wall-time limit
-// ends a wait first.
+// A poll suspends in hardware for up to a system-dependent time; the wall-time limit ends a wait
+// first.
 constexpr uint32_t kSpinLimit = 1u << 24;
 constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s
 
@@ -58,6 +58,10 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
                  "r"(bytes)
                  : "memory");
 }
+// Adds `bytes` to what the current phase waits for, without an arrival.
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
+    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -69,21 +73,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait for the phase with the given parity to complete. On timeout, records `code` in
-// *err (first error wins) and returns false.
-// try_wait with a suspend-time hint: the thread sleeps in hardware (up to `ns`) until the phase
-// completes, instead of spinning through instruction issue.
-__device__ __forceinline__ bool mbar_try_wait_hint(uint64_t* bar, uint32_t parity, uint32_t ns) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(ns)
-        : "memory");
-    return ok != 0;
-}
 __device__ __forceinline__ uint64_t global_ns() {
     uint64_t t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -91,15 +80,19 @@ __device__ __forceinline__ uint64_t global_ns() {
 }
 // Bounded wait for the phase with the given parity to complete: gives up after kWaitLimitNs of
 // wall time (or kSpinLimit polls), records `code` in *err (first error wins) and returns false.
-// Returns early without waiting when another wait has already recorded an error.
+// Returns early without waiting when another wait has already recorded an error. Polls carry no
+// suspend-time hint: with one the compiler adds a sleep loop whose instructions compete with the
+// working warps (brute-force kernel at 32768 x 32768: 235 us with a 1 us hint, 224 us without).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t* err, uint32_t code) {
     if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t t0 = global_ns();
+    uint64_t t0 = 0;  // the clock is read every 64 polls only: an ordinary wait ends before
     for (uint32_t i = 0; i < kSpinLimit; ++i) {
-        if (mbar_try_wait_hint(bar, parity, 1000u)) return true;
+        if (mbar_try_wait(bar, parity)) return true;
         if ((i & 63u) == 63u) {
             if (*reinterpret_cast<volatile uint32_t*>(err) != 0u) return false;
-            if (global_ns() - t0 > kWaitLimitNs) break;
+            const uint64_t now = global_ns();
+            if (t0 == 0) t0 = now;
+            if (now - t0 > kWaitLimitNs) break;
         }
     }
     atomicCAS(err, 0u, code);
@@ -191,6 +184,18 @@ __device__ __forceinline__ uint64_t umma_desc_k_sw128(uint32_t smem_addr) {
     return d;
 }
 
+// The same for 32-byte rows stored with the 32-byte swizzle (8-row atoms of 256 bytes; 16-byte chunk
+// c of row r at 32 r + 16 (c ^ (r / 4 % 2))): one K = 32 step of 8-bit elements. 256-byte aligned.
+__device__ __forceinline__ uint64_t umma_desc_k_sw32(uint32_t smem_addr) {
+    uint64_t d = 0;
+    d |= static_cast<uint64_t>((smem_addr >> 4) & 0x3FFFu);
+    d |= static_cast<uint64_t>(1u) << 16;
+    d |= static_cast<uint64_t>(256u >> 4) << 32;  // SBO: 8 rows x 32 B
+    d |= static_cast<uint64_t>(1u) << 46;
+    d |= static_cast<uint64_t>(6u) << 61;         // layout: 32-byte swizzle
+    return d;
+}
+
 // Instruction descriptor: kind::i8, A and B unsigned 8-bit, K-major both, D = s32.
 __host__ __device__ constexpr uint32_t idesc_u8u8_s32(int M, int N) {
     return (2u << 4)                                   // D format s32
@@ -224,6 +229,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
           "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
           "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
           "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+}
+// 16 consecutive columns.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
