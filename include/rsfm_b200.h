@@ -364,6 +364,13 @@ int rsfm_ranked_pack_records(const uint8_t* keys, const uint32_t* codes, const u
 int rsfm_ranked_pack_table_records(const uint32_t* records, const uint32_t* buckets, uint32_t nbDesc,
                                    uint32_t* tableRecords, cudaStream_t stream);
 
+/* rsfm_ranked_pack_table_records for images stored back to back, in the layout of
+ * rsfm_ranked_register_flat (no reference counterpart): image i's records at imageBegin[i], its
+ * lists and table records at 8 * imageBegin[i] (imageBegin: host array of nbImages + 1,
+ * imageBegin[0] = 0; each image below 2^24 descriptors). One launch per 960 images. */
+int rsfm_ranked_pack_table_records_flat(const uint32_t* records, const uint32_t* buckets, const uint32_t* imageBegin,
+                                        uint32_t nbImages, uint32_t* tableRecords, cudaStream_t stream);
+
 /* Ranked cascade-hash matching (no reference counterpart): for every query descriptor, the
  * candidates are the train descriptors sharing one of the first nbTables bucket keys; they are
  * ranked by Hamming distance of the codes (ties: lower index), the first topK (<= 32) are scored

@@ -224,6 +224,8 @@ SIGNATURES = {
     "rsfm_ranked_batch_destroy": (ctypes.c_int, [ctypes.c_void_p]),
     "rsfm_ranked_pack_records": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint32,
                                                 ctypes.c_void_p, ctypes.c_void_p]),
+    "rsfm_ranked_pack_table_records_flat": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
+                                                           ctypes.c_uint32, ctypes.c_void_p, ctypes.c_void_p]),
     "rsfm_ranked_pack_table_records": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint32,
                                                       ctypes.c_void_p, ctypes.c_void_p]),
     "rsfm_bf_plan_launch": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p]),

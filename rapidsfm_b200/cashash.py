@@ -105,7 +105,7 @@ def register_ranked_images(hasher, descs, stream=None, table_records=False):
     descriptors are first copied back to back into one buffer; every per-descriptor step then runs
     once over all of them and every bucket-build step once for all images. hasher: a CasHash with
     192 channels or a learned_hash.LearnedHash. table_records: also pack each image's records in
-    bucket-list order (RankedImage.pack_table_records, one launch per image; only train images use
+    bucket-list order (as RankedImage.pack_table_records, in one launch; only train images use
     them, and only images of fewer than 2^24 descriptors can have them). Returns one
     RankedImage per input (views of shared buffers, including the packed copy of its descriptors)."""
     lib = _lib.load()
@@ -134,16 +134,18 @@ def register_ranked_images(hasher, descs, stream=None, table_records=False):
     _lib.check(lib.rsfm_ranked_register_flat(ctypes.byref(h), _p(flat), begin, len(descs), _p(keys), _p(codes),
                                              _p(sqr), _p(upper), _p(maxb), _p(buckets), _p(records),
                                              _stream_ptr(stream)), "rsfm_ranked_register_flat")
-    imgs = []
-    for k, n in enumerate(ns):
-        o = int(offs[k])
-        imgs.append(RankedImage.from_parts(flat[o:o + n], keys[o:o + n], codes[o:o + n], sqr[o:o + n], upper[k],
-                                           maxb[k:k + 1], buckets[8 * o:8 * (o + n)].view(8, n), records[o:o + n]))
+    # views by split: one call per buffer instead of several per image
+    imgs = [RankedImage.from_parts(*parts[:6], parts[6].view(8, n), parts[7])
+            for n, *parts in zip(ns, flat[:total].split(ns), keys[:total].split(ns), codes[:total].split(ns),
+                                 sqr[:total].split(ns), upper.unbind(0), maxb.split(1),
+                                 buckets[:8 * total].split([8 * n for n in ns]), records[:total].split(ns))]
     if table_records:
         trec = torch.empty((8 * cap, 8), dtype=torch.int32, device=dev)
-        for k, img in enumerate(imgs):
-            o = int(offs[k])
-            img.pack_table_records(out=trec[8 * o:8 * (o + img.n)] if img.n else trec[:8], stream=stream)
+        _lib.check(lib.rsfm_ranked_pack_table_records_flat(_p(records), _p(buckets), begin, len(descs), _p(trec),
+                                                           _stream_ptr(stream)),
+                   "rsfm_ranked_pack_table_records_flat")
+        for img, out in zip(imgs, trec[:8 * total].split([8 * n for n in ns])):
+            img.table_records = out if img.n else trec[:8]
     return imgs
 
 

@@ -132,3 +132,20 @@ def test_pack_table_records_arguments_checked_without_gpu(rsfm):
     assert pack(None, 0x20000, 100, 0x30000, None) == 1
     assert pack(0x10000, None, 100, 0x30000, None) == 1
     assert pack(0x10000, 0x20000, 1 << 24, 0x30000, None) == 1
+
+
+def test_pack_table_records_flat_arguments_checked_without_gpu(rsfm):
+    """rsfm_ranked_pack_table_records_flat: no images or only empty ones is nothing to do; begins that
+    fall or do not start at 0, an image of 2^24 descriptors, missing or misaligned buffers are refused."""
+    import ctypes
+    pack = rsfm._lib.load().rsfm_ranked_pack_table_records_flat
+
+    def call(begin, rec=32, buckets=64, out=96):
+        arr = (ctypes.c_uint32 * len(begin))(*begin)
+        return pack(rec, buckets, arr, len(begin) - 1, out, None)
+
+    assert pack(None, None, None, 0, None, None) == 0
+    assert call([0, 0, 0], None, None, None) == 0
+    for bad in ([1, 2], [0, 5, 4], [0, 1 << 24]):
+        assert call(bad) == 1
+    assert call([0, 4], rec=None) == 1 and call([0, 4], rec=16) == 1 and call([0, 4], out=48) == 1

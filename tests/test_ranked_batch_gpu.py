@@ -343,3 +343,20 @@ def test_cascade_matcher_table_records_same_results(rsfm):
     torch.cuda.synchronize()
     for a, b in zip(*got):
         assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("sizes", [[1], [0, 3, 0, 255, 257, 1], [2047, 2049, 300], [5, 0, 7] * 400])
+def test_flat_table_records_equal_per_image_packing(rsfm, sizes):
+    """Images packed in one launch (blocks of 2048 entries cross image borders; more than 960 images
+    take a second launch; empty images) against rsfm_ranked_pack_table_records image by image."""
+    from rapidsfm_b200 import cashash as ch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(len(sizes))
+    descs = [torch.randint(0, 256, (n, 128), dtype=torch.uint8, device="cuda", generator=g) for n in sizes]
+    cas = ch.CasHash(ch.gaussian_weights(3))
+    imgs = ch.register_ranked_images(cas, descs, table_records=True)
+    for img, n in zip(imgs, sizes):
+        got = img.table_records[:8 * n].clone()
+        want = torch.full((8 * max(n, 1), 8), -7, dtype=torch.int32, device="cuda")
+        img.pack_table_records(out=want)
+        assert torch.equal(got, want[:8 * n])
