@@ -67,3 +67,29 @@ def test_batch_equals_single(rsfm, oracle):
     assert rsfm.last_launch_count() == 2
     for t, e in zip(tasks, expect):
         np.testing.assert_array_equal(t["votes"].cpu().numpy()[:len(e)], e)
+
+
+@pytest.mark.parametrize("n", [16, 17, 129, 1023, 1025])
+def test_odd_counts_and_stage_edge(rsfm, oracle, n):
+    """Matches are tested two at a time: odd neighbourhood sizes (one cell holds them all), one short
+    of, at and past the 1024 staged matches, next to an empty pair whose votes must come out zero."""
+    rng = np.random.default_rng(n)
+    m, _ = synth.make_ransac_matches(n, inlier_frac=0.7, seed=n, cluster=(55.0, 55.0, 40.0))
+    few = rng.uniform(0, 100, (7, 4)).astype(np.float32)
+    tasks = []
+    for x in (m, few):
+        sp, bounds, _, cols, rows, cw = ransac.bin_matches(1600, 1200, x)
+        votes, aff = ransac.device_buffers(len(sp), cols, rows)
+        votes.fill_(99)
+        tasks.append((sp, bounds, cols, rows, float(np.float32(cw) * np.float32(0.15)), votes, aff))
+    for mode in (0, 1, 2):
+        dev = [dict(votes=v, affines=a, matches=torch.from_numpy(sp).cuda(),
+                    bounds=torch.from_numpy(b.view(np.int32)).cuda(), cols=c, rows=r, threshold=t)
+               for sp, b, c, r, t, v, a in tasks]
+        ransac.ransac_match_filter_batch(dev, try_other=mode, seed=5)
+        torch.cuda.synchronize()
+        sp, b, c, r, t, v, a = tasks[0]
+        eaff, evotes = oracle.ransac_votes(sp, b, c, r, 256, t, mode, 5)
+        np.testing.assert_array_equal(v.cpu().numpy()[:n], evotes[:n])
+        np.testing.assert_array_equal(a.cpu().numpy().view(np.uint32).ravel(), eaff.view(np.uint32).ravel())
+        assert int(tasks[1][5].sum()) == 0
