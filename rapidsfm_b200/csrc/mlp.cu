@@ -255,14 +255,17 @@ infer_kernel(const uint16_t* __restrict__ w1, const float* __restrict__ b1, cons
 // weight gradients need, so every operand is K-major. TMA loads 64-element K panels (128-byte
 // swizzle) of A (128 rows) and B (N rows) into a kGStages-deep ring. One 128-row M tile per CTA
 // (blockIdx.x) and one K range per CTA (blockIdx.y: split-K); N (128 or 256) is the whole width.
-// Warp 0 = TMA producer, warp 1 = TMEM allocator and MMA issuer, warps 2-5 = epilogue (TMEM lane
-// quarter warp % 4, one output row per thread, 32 columns per TMEM load).
+// Warp 0 = TMA producer, warp 1 = TMEM allocator and MMA issuer, warps 2-9 = epilogue (TMEM lane
+// quarter warp % 4, one output row per thread, 32 columns per TMEM load; each of the two warps of a
+// quarter takes half of the columns: these GEMMs have two to six K steps, so the epilogue's stores
+// are most of a launch).
 constexpr int kGStages = 4;
-constexpr int kGThreads = 192;
+constexpr int kGEpi = 8;  // epilogue warps: two per TMEM lane quarter, each half of the columns
+constexpr int kGThreads = 32 * (2 + kGEpi);
 enum GemmEpi : int {
     kEpiStoreF32 = 0,      // outF[m][n] = d
     kEpiBiasReluBf16 = 1,  // h = bf16(relu(d + bias[n])) into outB[m][n] and outT[n][m]
-    kEpiReluGrad = 2,      // g = d * [mask[m][n] > 0] into outF[m][n] (fp32) and outT[n][m] (bf16)
+    kEpiReluGrad = 2,      // g = d * [mask[m][n] > 0] into outT[n][m] (bf16), its fp32 column sums added to outF[n]
     kEpiAtomicF32 = 3,     // outF[m][n] += d (split-K partial sums into a zeroed outF)
 };
 struct GemmArgs {
@@ -344,11 +347,13 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_tc_kernel(const __grid_cons
         const uint32_t q = warp & 3u, m = m0 + 32u * q + lane;
         mbar_wait(&S.done, 0, G.err, kDevTimeoutAccFull);
         tc_fence_after();
-        for (uint32_t c0 = 0; c0 < G.N; c0 += 32u) {
+        const uint32_t cBegin = (warp - 2u) / 4u * (G.N / 2u), cEnd = cBegin + G.N / 2u;
+        for (uint32_t c0 = cBegin; c0 < cEnd; c0 += 32u) {
             uint32_t v[32];
             tmem_ld32(tmem + ((32u * q) << 16) + c0, v);
             tmem_wait_ld();
-            if (m >= G.M) continue;  // (after the warp-collective load)
+            const bool in = m < G.M;
+            if (!in && G.epi != kEpiReluGrad) continue;  // (after the warp-collective load)
             float f[32];
 #pragma unroll
             for (int k = 0; k < 32; ++k) f[k] = __uint_as_float(v[k]);
@@ -374,15 +379,26 @@ __global__ void __launch_bounds__(kGThreads, 1) gemm_tc_kernel(const __grid_cons
                     const uint4* mk = reinterpret_cast<const uint4*>(G.mask + size_t(m) * G.ldMask + c0);
                     uint16_t mb[32];
 #pragma unroll
-                    for (int k4 = 0; k4 < 4; ++k4) *reinterpret_cast<uint4*>(&mb[8 * k4]) = mk[k4];
+                    for (int k4 = 0; k4 < 4; ++k4)
+                        *reinterpret_cast<uint4*>(&mb[8 * k4]) = in ? mk[k4] : make_uint4(0, 0, 0, 0);
+                    // Column sums of the fp32 values (a bias gradient): each warp turns its 32 x 32
+                    // block through shared memory (the operand stages, free once the MMAs are done)
+                    // and each lane adds up one column. Writing the values out and summing them in a
+                    // kernel of its own took 8 us more a step at batch 4096.
+                    float* tr = reinterpret_cast<float*>(S.a[0]) + (warp - 2u) * (32u * 33u);
 #pragma unroll
                     for (int k = 0; k < 32; ++k) {
                         if (!(bf16_to_f(mb[k]) > 0.f)) f[k] = 0.f;
                         hb[k] = bf16_bits(f[k]);
+                        tr[lane * 33u + uint32_t(k)] = f[k];
                     }
-                    float4* o = reinterpret_cast<float4*>(G.outF + size_t(m) * G.ldF + c0);
+                    __syncwarp();
+                    float sum = 0.f;
 #pragma unroll
-                    for (int k4 = 0; k4 < 8; ++k4) o[k4] = make_float4(f[4 * k4], f[4 * k4 + 1], f[4 * k4 + 2], f[4 * k4 + 3]);
+                    for (int r = 0; r < 32; ++r) sum += tr[uint32_t(r) * 33u + lane];
+                    atomicAdd(&G.outF[c0 + lane], sum);
+                    __syncwarp();
+                    if (!in) continue;
                 }
                 // transposed copy: per column, the warp's 32 consecutive rows (64 contiguous bytes)
 #pragma unroll
@@ -418,19 +434,33 @@ __global__ void gather_convert_kernel(const uint8_t* __restrict__ da, const uint
     for (int k = 0; k < 16; ++k) xT[size_t(16 * g + k) * ldT + r] = o[k];
 }
 
-// out[c][r] = bf16(in[r][c]) for in f32 [rows][cols] (32 x 32 tiles through shared memory).
+// out[c][r] = bf16(in[r][c]) for in f32 [rows][cols] (32 x 32 tiles through shared memory, kTrTiles of
+// them down a block's rows); with `sums`, sums[c] += sum_r in[r][c] too (one read for both).
+constexpr uint32_t kTrTiles = 4;
 __global__ void transpose_bf16_kernel(const float* __restrict__ in, uint32_t rows, uint32_t cols,
-                                      uint16_t* __restrict__ out, uint32_t ldOut) {
+                                      uint16_t* __restrict__ out, uint32_t ldOut, float* __restrict__ sums) {
     __shared__ float t[32][33];
-    const uint32_t r0 = blockIdx.y * 32u, c0 = blockIdx.x * 32u;
-    for (uint32_t y = threadIdx.y; y < 32u; y += blockDim.y) {
-        const uint32_t r = r0 + y, c = c0 + threadIdx.x;
-        t[y][threadIdx.x] = (r < rows && c < cols) ? in[size_t(r) * cols + c] : 0.f;
+    const uint32_t c0 = blockIdx.x * 32u, cx = c0 + threadIdx.x;
+    float sum = 0.f;
+    for (uint32_t r0 = blockIdx.y * 32u * kTrTiles, e = min(rows, r0 + 32u * kTrTiles); r0 < e; r0 += 32u) {
+        for (uint32_t y = threadIdx.y; y < 32u; y += blockDim.y) {
+            const float v = (r0 + y < rows && cx < cols) ? in[size_t(r0 + y) * cols + cx] : 0.f;
+            t[y][threadIdx.x] = v;
+            sum += v;
+        }
+        __syncthreads();
+        for (uint32_t y = threadIdx.y; y < 32u; y += blockDim.y) {
+            const uint32_t c = c0 + y, r = r0 + threadIdx.x;
+            if (c < cols && r < rows) out[size_t(c) * ldOut + r] = bf16_bits(t[threadIdx.x][y]);
+        }
+        __syncthreads();
     }
+    if (!sums) return;
+    t[threadIdx.y][threadIdx.x] = sum;
     __syncthreads();
-    for (uint32_t y = threadIdx.y; y < 32u; y += blockDim.y) {
-        const uint32_t c = c0 + y, r = r0 + threadIdx.x;
-        if (c < cols && r < rows) out[size_t(c) * ldOut + r] = bf16_bits(t[threadIdx.x][y]);
+    if (threadIdx.y == 0 && cx < cols) {
+        for (uint32_t y = 1; y < blockDim.y; ++y) sum += t[y][threadIdx.x];
+        atomicAdd(&sums[cx], sum);
     }
 }
 
@@ -494,17 +524,6 @@ __global__ void triplet_kernel(const float* __restrict__ o, const float* __restr
     dOb[size_t(2 * B + b) * 128 + c] = bf16_bits(on);
     if (lossKey != 0.f) atomicAdd(lossSum, lossKey * inv);
     if (c == 0 && active) atomicAdd(lossSum, l * inv);
-}
-
-// column sums: out[c] += sum_r in[r][c] (out zeroed beforehand); block = one thread per column,
-// kColRows rows per block, one atomic per column per block.
-constexpr uint32_t kColRows = 128;
-__global__ void colsum_kernel(const float* __restrict__ in, uint32_t rows, uint32_t cols, float* __restrict__ out) {
-    const uint32_t c = threadIdx.x;
-    const uint32_t r0 = blockIdx.x * kColRows, r1 = min(rows, r0 + kColRows);
-    float s = 0.f;
-    for (uint32_t r = r0; r < r1; ++r) s += in[size_t(r) * cols + c];
-    atomicAdd(&out[c], s);
 }
 
 // Adam on fp32 masters; writes the bf16 copy when `bf` is non-null.
@@ -591,7 +610,7 @@ struct rsfm_mlp_trainer {
     // [columns][ldR], the K-major operands of the weight-gradient GEMMs
     uint16_t *xb = nullptr, *xT = nullptr;         // bf16 x / 64
     uint16_t *h = nullptr, *hT = nullptr;          // bf16 relu(x W1^T + b1) [R][256]
-    float *o = nullptr, *dO = nullptr, *dh = nullptr, *loss = nullptr;
+    float *o = nullptr, *dO = nullptr, *loss = nullptr;
     uint16_t *dOb = nullptr, *dOT = nullptr, *dhT = nullptr;
     uint16_t *bw1 = nullptr, *bw2 = nullptr;  // bf16 copies the hash kernel reads
     uint16_t* w2T = nullptr;                  // bf16 W2^T [256][128] (the B operand of dh = dO W2)
@@ -644,7 +663,7 @@ extern "C" int rsfm_mlp_trainer_create(const float* initParams, uint32_t batch, 
               cudaMalloc(&t->xT, 128 * L * 2) == cudaSuccess && cudaMalloc(&t->h, R * 256 * 2) == cudaSuccess &&
               cudaMalloc(&t->hT, 256 * L * 2) == cudaSuccess && cudaMalloc(&t->o, R * 128 * 4) == cudaSuccess &&
               cudaMalloc(&t->dO, R * 128 * 4) == cudaSuccess && cudaMalloc(&t->dOb, R * 128 * 2) == cudaSuccess &&
-              cudaMalloc(&t->dOT, 128 * L * 2) == cudaSuccess && cudaMalloc(&t->dh, R * 256 * 4) == cudaSuccess &&
+              cudaMalloc(&t->dOT, 128 * L * 2) == cudaSuccess &&
               cudaMalloc(&t->dhT, 256 * L * 2) == cudaSuccess && cudaMalloc(&t->loss, 4) == cudaSuccess &&
               cudaMalloc(&t->bw1, kNW1 * 2) == cudaSuccess && cudaMalloc(&t->bw2, kNW2 * 2) == cudaSuccess &&
               cudaMalloc(&t->w2T, kNW2 * 2) == cudaSuccess && cudaMalloc(&t->stepDev, 4) == cudaSuccess;
@@ -665,7 +684,7 @@ extern "C" int rsfm_mlp_trainer_create(const float* initParams, uint32_t batch, 
     }
     mlp::f32_to_bf16_kernel<<<(kNW1 + 255) / 256, 256>>>(t->w1, t->bw1, kNW1);
     mlp::f32_to_bf16_kernel<<<(kNW2 + 255) / 256, 256>>>(t->w2, t->bw2, kNW2);
-    mlp::transpose_bf16_kernel<<<dim3(256 / 32, 128 / 32), dim3(32, 8)>>>(t->w2, 128, 256, t->w2T, 128);
+    mlp::transpose_bf16_kernel<<<dim3(256 / 32, 1), dim3(32, 8)>>>(t->w2, 128, 256, t->w2T, 128, nullptr);
     if (cudaDeviceSynchronize() != cudaSuccess) {
         rsfm_mlp_trainer_destroy(t);
         return RSFM_ERR_CUDA;
@@ -693,8 +712,7 @@ extern "C" int rsfm_mlp_trainer_create(const float* initParams, uint32_t batch, 
     if (st == RSFM_OK) {
         G[2].mask = t->h;
         G[2].ldMask = 256;
-        G[2].outF = t->dh;
-        G[2].ldF = 256;
+        G[2].outF = t->g + kNW1;  // db1
         G[2].outT = t->dhT;
         G[2].ldT = t->ldR;
         st = gemm_args(&G[3], t->dOT, t->ldR, t->hT, t->ldR, 128, 256, Ru, kSplit, kEpiAtomicF32);  // dW2 = dO^T h
@@ -744,23 +762,20 @@ static int trainer_grads(rsfm_mlp_trainer* t, const void* a, const uint32_t* ia,
     RSFM_CUDA_TRY(cudaGetLastError());
     RSFM_CUDA_TRY(cudaMemsetAsync(t->g, 0, kNP * 4, s));
     RSFM_CUDA_TRY(cudaMemsetAsync(t->loss, 0, 4, s));
-    float* gB1 = t->g + kNW1;
     float* gB2 = t->g + kNW1 + kNB1 + kNW2;
     int st = gemm_tc(s, t->gemm[0]);  // h, h^T = bf16(relu(x W1^T + b1))
     if (st == RSFM_OK) st = gemm_tc(s, t->gemm[1]);  // o = h W2^T
     if (st != RSFM_OK) return st;
     triplet_kernel<<<B, 128, 0, s>>>(t->o, t->model.b2, t->dO, t->dOb, B, t->margin, t->kind, t->lambda, t->loss);
-    transpose_bf16_kernel<<<dim3(128 / 32, (R + 31) / 32), dim3(32, 8), 0, s>>>(t->dO, R, 128, t->dOT, t->ldR);
-    colsum_kernel<<<(R + kColRows - 1) / kColRows, 128, 0, s>>>(t->dO, R, 128, gB2);  // db2 = sum dO
+    transpose_bf16_kernel<<<dim3(128 / 32, (R + 32 * kTrTiles - 1) / (32 * kTrTiles)), dim3(32, 8), 0, s>>>(
+        t->dO, R, 128, t->dOT, t->ldR, gB2);  // dO^T, db2 = sum dO
     RSFM_CUDA_TRY(cudaGetLastError());
-    st = gemm_tc(s, t->gemm[2]);  // dh, dh^T = (dO W2) [h > 0]
+    st = gemm_tc(s, t->gemm[2]);  // dh^T = ((dO W2) [h > 0])^T, db1 = sum dh
     if (st != RSFM_OK) return st;
-    colsum_kernel<<<(R + kColRows - 1) / kColRows, 256, 0, s>>>(t->dh, R, 256, gB1);  // db1 = sum dh
-    RSFM_CUDA_TRY(cudaGetLastError());
     st = gemm_tc(s, t->gemm[3]);  // dW2 += dO^T h (split-K)
     if (st == RSFM_OK) st = gemm_tc(s, t->gemm[4]);  // dW1 += dh^T (x / 64) (split-K)
     if (st != RSFM_OK) return st;
-    launch_count_add(5);
+    launch_count_add(3);
     return RSFM_OK;
 }
 
@@ -789,7 +804,7 @@ extern "C" int rsfm_mlp_trainer_step(rsfm_mlp_trainer* t, const void* a, const u
     adam_all_kernel<<<(kNP + 255) / 256, 256, 0, stream>>>(t->w1, t->g, t->m1, t->m2, t->bw1, t->bw2, kNW1, kNB1,
                                                           kNW2, kNB2, t->lr, t->stepDev);
     step_increment_kernel<<<1, 1, 0, stream>>>(t->stepDev);
-    transpose_bf16_kernel<<<dim3(256 / 32, 128 / 32), dim3(32, 8), 0, stream>>>(t->w2, 128, 256, t->w2T, 128);
+    transpose_bf16_kernel<<<dim3(256 / 32, 1), dim3(32, 8), 0, stream>>>(t->w2, 128, 256, t->w2T, 128, nullptr);
     RSFM_CUDA_TRY(cudaGetLastError());
     launch_count_add(3);
     if (lossDevice) RSFM_CUDA_TRY(cudaMemcpyAsync(lossDevice, t->loss, 4, cudaMemcpyDeviceToDevice, stream));
@@ -808,7 +823,7 @@ extern "C" int rsfm_mlp_trainer_destroy(rsfm_mlp_trainer* t) {
                     static_cast<void*>(t->m2), static_cast<void*>(t->xb),
                     static_cast<void*>(t->xT), static_cast<void*>(t->h), static_cast<void*>(t->hT),
                     static_cast<void*>(t->o), static_cast<void*>(t->dO), static_cast<void*>(t->dOb),
-                    static_cast<void*>(t->dOT), static_cast<void*>(t->dh), static_cast<void*>(t->dhT),
+                    static_cast<void*>(t->dOT), static_cast<void*>(t->dhT),
                     static_cast<void*>(t->loss), static_cast<void*>(t->bw1), static_cast<void*>(t->bw2),
                     static_cast<void*>(t->w2T), static_cast<void*>(t->stepDev)})
         if (p) cudaFree(p);
