@@ -435,11 +435,14 @@ __global__ void gather_convert_kernel(const uint8_t* __restrict__ da, const uint
 }
 
 // out[c][r] = bf16(in[r][c]) for in f32 [rows][cols] (32 x 32 tiles through shared memory, kTrTiles of
-// them down a block's rows); with `sums`, sums[c] += sum_r in[r][c] too (one read for both).
+// them down a block's rows); with `sums`, sums[c] += sum_r in[r][c] too (one read for both); with `step`,
+// the step counter that the kernel before read is advanced (a launch of its own took 1.1 us).
 constexpr uint32_t kTrTiles = 4;
 __global__ void transpose_bf16_kernel(const float* __restrict__ in, uint32_t rows, uint32_t cols,
-                                      uint16_t* __restrict__ out, uint32_t ldOut, float* __restrict__ sums) {
+                                      uint16_t* __restrict__ out, uint32_t ldOut, float* __restrict__ sums,
+                                      uint32_t* __restrict__ step) {
     __shared__ float t[32][33];
+    if (step && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) *step += 1u;
     const uint32_t c0 = blockIdx.x * 32u, cx = c0 + threadIdx.x;
     float sum = 0.f;
     for (uint32_t r0 = blockIdx.y * 32u * kTrTiles, e = min(rows, r0 + 32u * kTrTiles); r0 < e; r0 += 32u) {
@@ -551,8 +554,6 @@ __global__ void adam_all_kernel(float* __restrict__ w, const float* __restrict__
     if (x >= o2 && x < o2 + nW2) bw2[x - o2] = *reinterpret_cast<const uint16_t*>(&bv);
 }
 
-__global__ void step_increment_kernel(uint32_t* step) { *step += 1u; }
-
 __global__ void f32_to_bf16_kernel(const float* __restrict__ in, uint16_t* __restrict__ out, uint32_t n) {
     const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x < n) {
@@ -657,14 +658,14 @@ extern "C" int rsfm_mlp_trainer_create(const float* initParams, uint32_t batch, 
     const size_t R = size_t(3) * batch;
     t->ldR = uint32_t((R + 7) & ~size_t(7));
     const size_t L = t->ldR;
-    bool ok = cudaMalloc(&t->w1, kNP * 4) == cudaSuccess && cudaMalloc(&t->g, kNP * 4) == cudaSuccess &&
+    bool ok = cudaMalloc(&t->w1, kNP * 4) == cudaSuccess && cudaMalloc(&t->g, (kNP + 1) * 4) == cudaSuccess &&
               cudaMalloc(&t->m1, kNP * 4) == cudaSuccess && cudaMalloc(&t->m2, kNP * 4) == cudaSuccess &&
               cudaMalloc(&t->xb, R * 128 * 2) == cudaSuccess &&
               cudaMalloc(&t->xT, 128 * L * 2) == cudaSuccess && cudaMalloc(&t->h, R * 256 * 2) == cudaSuccess &&
               cudaMalloc(&t->hT, 256 * L * 2) == cudaSuccess && cudaMalloc(&t->o, R * 128 * 4) == cudaSuccess &&
               cudaMalloc(&t->dO, R * 128 * 4) == cudaSuccess && cudaMalloc(&t->dOb, R * 128 * 2) == cudaSuccess &&
               cudaMalloc(&t->dOT, 128 * L * 2) == cudaSuccess &&
-              cudaMalloc(&t->dhT, 256 * L * 2) == cudaSuccess && cudaMalloc(&t->loss, 4) == cudaSuccess &&
+              cudaMalloc(&t->dhT, 256 * L * 2) == cudaSuccess &&
               cudaMalloc(&t->bw1, kNW1 * 2) == cudaSuccess && cudaMalloc(&t->bw2, kNW2 * 2) == cudaSuccess &&
               cudaMalloc(&t->w2T, kNW2 * 2) == cudaSuccess && cudaMalloc(&t->stepDev, 4) == cudaSuccess;
     if (!ok) {
@@ -672,6 +673,7 @@ extern "C" int rsfm_mlp_trainer_create(const float* initParams, uint32_t batch, 
         return RSFM_ERR_CUDA;
     }
     t->w2 = t->w1 + kNW1 + kNB1;
+    t->loss = t->g + kNP;
     t->model.w1 = t->bw1;
     t->model.b1 = t->w1 + kNW1;
     t->model.w2 = t->bw2;
@@ -684,7 +686,7 @@ extern "C" int rsfm_mlp_trainer_create(const float* initParams, uint32_t batch, 
     }
     mlp::f32_to_bf16_kernel<<<(kNW1 + 255) / 256, 256>>>(t->w1, t->bw1, kNW1);
     mlp::f32_to_bf16_kernel<<<(kNW2 + 255) / 256, 256>>>(t->w2, t->bw2, kNW2);
-    mlp::transpose_bf16_kernel<<<dim3(256 / 32, 1), dim3(32, 8)>>>(t->w2, 128, 256, t->w2T, 128, nullptr);
+    mlp::transpose_bf16_kernel<<<dim3(256 / 32, 1), dim3(32, 8)>>>(t->w2, 128, 256, t->w2T, 128, nullptr, nullptr);
     if (cudaDeviceSynchronize() != cudaSuccess) {
         rsfm_mlp_trainer_destroy(t);
         return RSFM_ERR_CUDA;
@@ -760,15 +762,14 @@ static int trainer_grads(rsfm_mlp_trainer* t, const void* a, const uint32_t* ia,
                                                         static_cast<const uint8_t*>(ng), in_, B, t->xb, t->xT,
                                                         t->ldR);
     RSFM_CUDA_TRY(cudaGetLastError());
-    RSFM_CUDA_TRY(cudaMemsetAsync(t->g, 0, kNP * 4, s));
-    RSFM_CUDA_TRY(cudaMemsetAsync(t->loss, 0, 4, s));
+    RSFM_CUDA_TRY(cudaMemsetAsync(t->g, 0, (kNP + 1) * 4, s));  // gradients and the loss behind them
     float* gB2 = t->g + kNW1 + kNB1 + kNW2;
     int st = gemm_tc(s, t->gemm[0]);  // h, h^T = bf16(relu(x W1^T + b1))
     if (st == RSFM_OK) st = gemm_tc(s, t->gemm[1]);  // o = h W2^T
     if (st != RSFM_OK) return st;
     triplet_kernel<<<B, 128, 0, s>>>(t->o, t->model.b2, t->dO, t->dOb, B, t->margin, t->kind, t->lambda, t->loss);
     transpose_bf16_kernel<<<dim3(128 / 32, (R + 32 * kTrTiles - 1) / (32 * kTrTiles)), dim3(32, 8), 0, s>>>(
-        t->dO, R, 128, t->dOT, t->ldR, gB2);  // dO^T, db2 = sum dO
+        t->dO, R, 128, t->dOT, t->ldR, gB2, nullptr);  // dO^T, db2 = sum dO
     RSFM_CUDA_TRY(cudaGetLastError());
     st = gemm_tc(s, t->gemm[2]);  // dh^T = ((dO W2) [h > 0])^T, db1 = sum dh
     if (st != RSFM_OK) return st;
@@ -803,10 +804,9 @@ extern "C" int rsfm_mlp_trainer_step(rsfm_mlp_trainer* t, const void* a, const u
     using namespace mlp;
     adam_all_kernel<<<(kNP + 255) / 256, 256, 0, stream>>>(t->w1, t->g, t->m1, t->m2, t->bw1, t->bw2, kNW1, kNB1,
                                                           kNW2, kNB2, t->lr, t->stepDev);
-    step_increment_kernel<<<1, 1, 0, stream>>>(t->stepDev);
-    transpose_bf16_kernel<<<dim3(256 / 32, 1), dim3(32, 8), 0, stream>>>(t->w2, 128, 256, t->w2T, 128, nullptr);
+    transpose_bf16_kernel<<<dim3(256 / 32, 1), dim3(32, 8), 0, stream>>>(t->w2, 128, 256, t->w2T, 128, nullptr, t->stepDev);
     RSFM_CUDA_TRY(cudaGetLastError());
-    launch_count_add(3);
+    launch_count_add(2);
     if (lossDevice) RSFM_CUDA_TRY(cudaMemcpyAsync(lossDevice, t->loss, 4, cudaMemcpyDeviceToDevice, stream));
     return RSFM_OK;
 }
@@ -824,7 +824,7 @@ extern "C" int rsfm_mlp_trainer_destroy(rsfm_mlp_trainer* t) {
                     static_cast<void*>(t->xT), static_cast<void*>(t->h), static_cast<void*>(t->hT),
                     static_cast<void*>(t->o), static_cast<void*>(t->dO), static_cast<void*>(t->dOb),
                     static_cast<void*>(t->dOT), static_cast<void*>(t->dhT),
-                    static_cast<void*>(t->loss), static_cast<void*>(t->bw1), static_cast<void*>(t->bw2),
+                    static_cast<void*>(t->bw1), static_cast<void*>(t->bw2),
                     static_cast<void*>(t->w2T), static_cast<void*>(t->stepDev)})
         if (p) cudaFree(p);
     delete t;

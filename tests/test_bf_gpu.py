@@ -143,3 +143,71 @@ def test_uniform_large_exact(rsfm, oracle):
     a = synth.uniform_bytes(12288, 21)
     b = synth.uniform_bytes(9000, 22)
     _check(oracle, a, b, _run_ext(rsfm, [(a, b)])[0])
+
+
+def _norm_spread(n, seed):
+    """SIFT-like rows among all-zero, all-127 and (odd seeds) all-255 and all-128 ones: norms beyond
+    what the norm digits hold, and units that may and may not be doubled (a byte above 127)."""
+    d = np.minimum(synth.make_pair(n, 1, 0.0, 1.0, seed=seed)[0], 127)
+    d[::97] = 0
+    d[5::89] = 127
+    if seed % 2:
+        d[3::83] = 255
+        d[7::101] = 128
+    return d
+
+
+@pytest.mark.parametrize("na,nb", [(1, 17), (15, 16), (127, 128), (128, 129), (255, 257), (256, 256), (257, 511),
+                                   (513, 4097), (64, 9000), (2500, 300)])
+@pytest.mark.parametrize("seed", [2, 3])
+def test_unit_and_chunk_edges(rsfm, oracle, na, nb, seed):
+    # Around the 16-value chunks, 128-row halves, 256-row units and 256-column blocks; norms outside
+    # the digits' range (residuals) and both kinds of units (doubled rows, rows with large bytes).
+    a, b = _norm_spread(na, seed), _norm_spread(nb, seed + 2)
+    _check(oracle, a, b, _run_ext(rsfm, [(a, b)])[0])
+
+
+@pytest.mark.parametrize("sizes", [[(700, 900), (300, 0), (0, 40), (1000, 20)], [(9000, 9100), (30, 8000)]])
+def test_phases_in_one_launch_and_apart(rsfm, oracle, sizes):
+    # Up to eight 256 x 256 blocks per SM a call is init + one cooperative launch; above, index
+    # resolution and flags are launches of their own. Same results, both entry points, empty sides.
+    pairs = []
+    for k, (na, nb) in enumerate(sizes):
+        q, t, _ = synth.make_pair(max(na, 1), max(nb, 1), 0.5, 8.0, seed=500 + k)
+        pairs.append((q[:na], t[:nb]))
+    tasks = [rsfm.BFTask(_dev(a), _dev(b)) for a, b in pairs]
+    rsfm.bf_match_ext(tasks)
+    assert rsfm.last_launch_count() == (2 if len(sizes) == 4 else 4)
+    got = _run_ext(rsfm, pairs)
+    rsfm.bf_match(tasks)
+    for (a, b), g, t in zip(pairs, got, tasks):
+        if len(a) and len(b):
+            _check(oracle, a, b, g)
+        else:
+            assert (g[0] == 0xFFFFFFFF).all() and (g[1] == 0xFFFFFFFF).all() and (g[3] == 0).all()
+        np.testing.assert_array_equal(np.stack(rsfm.unpack_best(t.bestA), 1), g[0])
+        np.testing.assert_array_equal(np.stack(rsfm.unpack_best(t.bestB), 1), g[1])
+
+
+def test_user_graph_capture_and_streams(rsfm, oracle):
+    # A caller's own graph around a small (cooperative) call, and calls on two streams at once.
+    pairs = [synth.make_pair(800, 1000, 0.5, 8.0, seed=40)[:2], synth.make_pair(1200, 600, 0.5, 8.0, seed=41)[:2]]
+    tasks = [rsfm.BFTask(_dev(a), _dev(b)) for a, b in pairs]
+    rsfm.bf_match_ext(tasks)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        rsfm.bf_match_ext([tasks[0]])
+    tasks[0].bestA.fill_(0)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for _ in range(5):
+        with torch.cuda.stream(streams[0]):
+            graph.replay()
+        rsfm.bf_match_ext([tasks[1]], stream=streams[1])
+    torch.cuda.synchronize()
+    assert rsfm.device_error() == 0
+    for (a, b), t in zip(pairs, tasks):
+        got = (np.stack(rsfm.unpack_best(t.bestA), 1), np.stack(rsfm.unpack_best(t.bestB), 1),
+               t.secondA.cpu().numpy().view(np.uint32), t.flagsA.cpu().numpy().view(np.uint32))
+        _check(oracle, a, b, got)
