@@ -84,8 +84,10 @@ struct alignas(64) TaskDev {
     uint32_t rowGroupBegin;
 };
 
-struct Params {
-    TaskDev tasks[kMaxTasksPerLaunch];
+// Launch parameters, with room for kTasks tasks: one (also for plans, whose tasks are in global memory)
+// or kMaxTasksPerLaunch. A launch copies its parameters: 7 KB for sixteen tasks cost a call of one
+// pair about 2 us of host time a launch.
+struct ParamsBase {
     const TaskDev* gtasks;  // when non-null: any number of tasks, in global memory
     uint32_t nTasks;
     uint32_t totalUnits;
@@ -95,18 +97,24 @@ struct Params {
     uint32_t unitBlocks;  // 256-column blocks per unit (<= 32: the chunk code holds 8 * 32 values)
     uint32_t* err;
 };
+template <int kTasks>
+struct Params : ParamsBase {
+    TaskDev tasks[kTasks];
+};
 
 struct Unit {
     uint32_t r0, c0, rows, cols;
 };
 
-__device__ __forceinline__ const TaskDev& task_of(const Params& P, uint32_t t) {
+template <int N>
+__device__ __forceinline__ const TaskDev& task_of(const Params<N>& P, uint32_t t) {
     return P.gtasks ? P.gtasks[t] : P.tasks[t];
 }
 
 // Unit u of task t, where t enters as the task of an earlier unit of this CTA (units are taken in
 // increasing order, so the search only moves forward).
-__device__ __forceinline__ Unit decode_unit(const Params& P, uint32_t u, uint32_t& t) {
+template <int N>
+__device__ __forceinline__ Unit decode_unit(const Params<N>& P, uint32_t u, uint32_t& t) {
     while (t + 1 < P.nTasks && task_of(P, t + 1).unitBegin <= u) ++t;
     const TaskDev& T = task_of(P, t);
     const uint32_t local = u - T.unitBegin;
@@ -274,7 +282,8 @@ __device__ __forceinline__ void resolve_item(const uint4* __restrict__ q, const 
 }
 
 // Last task at or after t whose `begin` is <= w (tasks without any share their successor's).
-__device__ __forceinline__ uint32_t task_at(const Params& P, uint32_t t, uint32_t TaskDev::*begin, uint32_t w) {
+template <int N>
+__device__ __forceinline__ uint32_t task_at(const Params<N>& P, uint32_t t, uint32_t TaskDev::*begin, uint32_t w) {
     uint32_t hi = P.nTasks - 1u;
     while (t < hi) {
         const uint32_t mid = (t + hi + 1u) >> 1;
@@ -285,7 +294,8 @@ __device__ __forceinline__ uint32_t task_at(const Params& P, uint32_t t, uint32_
 
 // Warp w0 of `warps` takes a run of consecutive groups of four results (rows of A, then columns of
 // B), eight lanes a result.
-__device__ __forceinline__ void resolve_phase(const Params& P, uint32_t w0, uint32_t warps, uint32_t lane) {
+template <int N>
+__device__ __forceinline__ void resolve_phase(const Params<N>& P, uint32_t w0, uint32_t warps, uint32_t lane) {
     const uint32_t l8 = lane & 7u;
     uint32_t t = 0;
     const uint32_t run = (P.totalGroups + warps - 1u) / warps, first = w0 * run;
@@ -305,7 +315,8 @@ __device__ __forceinline__ void resolve_phase(const Params& P, uint32_t w0, uint
 }
 
 // Flags of every row: bit0 ratio test, bit1 cross-check. Runs of 32-row groups as above.
-__device__ __forceinline__ void flags_phase(const Params& P, uint32_t w0, uint32_t warps, uint32_t lane) {
+template <int N>
+__device__ __forceinline__ void flags_phase(const Params<N>& P, uint32_t w0, uint32_t warps, uint32_t lane) {
     uint32_t t = 0;
     const uint32_t run = (P.totalRowGroups + warps - 1u) / warps, first = w0 * run;
     const uint32_t end = first < P.totalRowGroups ? min(P.totalRowGroups, first + run) : first;
@@ -327,8 +338,8 @@ __device__ __forceinline__ void flags_phase(const Params& P, uint32_t w0, uint32
 }
 
 // kSecond: the second-best distances are wanted too.
-template <bool kSecond>
-__global__ void __launch_bounds__(kThreads, 1) bf_match_kernel(const __grid_constant__ Params P) {
+template <bool kSecond, int N>
+__global__ void __launch_bounds__(kThreads, 1) bf_match_kernel(const __grid_constant__ Params<N> P) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     Smem& S = smem_aligned_1024<Smem>(smem_raw);
     const uint32_t warp = threadIdx.x >> 5;
@@ -671,10 +682,12 @@ __global__ void __launch_bounds__(kThreads, 1) bf_match_kernel(const __grid_cons
 }
 
 // The same two phases as launches of their own.
-__global__ void __launch_bounds__(256) bf_resolve_kernel(const __grid_constant__ Params P) {
+template <int N>
+__global__ void __launch_bounds__(256) bf_resolve_kernel(const __grid_constant__ Params<N> P) {
     resolve_phase(P, blockIdx.x * 8u + (threadIdx.x >> 5), gridDim.x * 8u, threadIdx.x & 31u);
 }
-__global__ void __launch_bounds__(256) bf_flags_kernel(const __grid_constant__ Params P) {
+template <int N>
+__global__ void __launch_bounds__(256) bf_flags_kernel(const __grid_constant__ Params<N> P) {
     flags_phase(P, blockIdx.x * 8u + (threadIdx.x >> 5), gridDim.x * 8u, threadIdx.x & 31u);
 }
 
@@ -736,46 +749,47 @@ static uint32_t choose_unit_blocks(const std::vector<std::pair<uint32_t, uint32_
     return pick;
 }
 
-template <bool kSecond>
+template <bool kSecond, int N>
 static int ensure_attr() {
-    return set_max_dynamic_smem(reinterpret_cast<const void*>(bf_match_kernel<kSecond>), sizeof(Smem) + 1024);
+    return set_max_dynamic_smem(reinterpret_cast<const void*>(bf_match_kernel<kSecond, N>), sizeof(Smem) + 1024);
 }
 
-// Up to eight blocks per SM a call is bound by its host time (2 us a launch), so matching, index
-// resolution and flags share one launch; beyond, the grid-wide barriers between them cost more than
-// launches (897 x 1013: 38 against 44 us a call; 32768 x 32768: 274 against 251 us).
-static bool fuse_phases(const Params& P, int nsm) {
-    return uint64_t(P.totalUnits) * P.unitBlocks <= uint64_t(nsm) * 8;
+// Up to eight blocks per SM, and results for one round of the resolving warps, a call is bound by its
+// host time (2 us and more a launch), so matching, index resolution and flags share one launch;
+// beyond, the grid-wide barriers between them cost more than launches (one launch against three, us
+// a call with all outputs: 4096 x 4096 47 and 57, 8192 x 8192 53.5 and 55, 10000 x 10000 68 and 56.5).
+static bool fuse_phases(const ParamsBase& P, int nsm) {
+    return uint64_t(P.totalUnits) * P.unitBlocks <= uint64_t(nsm) * 8 && P.totalGroups <= uint32_t(nsm) * 28u;
 }
 
 // The matcher and what follows it.
-template <bool kSecond>
-static int launch_match(const Params& P, int nsm, cudaStream_t stream) {
-    const int st = ensure_attr<kSecond>();
+template <bool kSecond, int N>
+static int launch_match(const Params<N>& P, int nsm, cudaStream_t stream) {
+    const int st = ensure_attr<kSecond, N>();
     if (st != RSFM_OK) return st;
     void* tok = nullptr;
     const bool prof = profile_begin(stream, &tok);
     if (P.fused) {
         // a CTA per unit, or enough for the results of a few units with many columns
         const uint32_t want = std::max(P.totalUnits, std::max(P.totalGroups, P.totalRowGroups) / (kThreads / 32) + 1);
-        void* args[] = {const_cast<Params*>(&P)};
-        RSFM_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(bf_match_kernel<kSecond>),
+        void* args[] = {const_cast<Params<N>*>(&P)};
+        RSFM_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(bf_match_kernel<kSecond, N>),
                                                   dim3(std::min<uint32_t>(want, uint32_t(nsm))), dim3(kThreads), args,
                                                   sizeof(Smem) + 1024, stream));
     } else if (P.totalUnits > 0) {
-        bf_match_kernel<kSecond><<<std::min<uint32_t>(P.totalUnits, uint32_t(nsm)), kThreads, sizeof(Smem) + 1024, stream>>>(P);
+        bf_match_kernel<kSecond, N><<<std::min<uint32_t>(P.totalUnits, uint32_t(nsm)), kThreads, sizeof(Smem) + 1024, stream>>>(P);
         RSFM_CUDA_TRY(cudaGetLastError());
     }
     if (prof) profile_end(stream, tok);
     launch_count_add(1);
     if (P.fused) return RSFM_OK;
     if (P.totalGroups > 0) {
-        bf_resolve_kernel<<<std::min<uint32_t>((P.totalGroups + 7) / 8, uint32_t(nsm) * 64u), 256, 0, stream>>>(P);
+        bf_resolve_kernel<N><<<std::min<uint32_t>((P.totalGroups + 7) / 8, uint32_t(nsm) * 64u), 256, 0, stream>>>(P);
         RSFM_CUDA_TRY(cudaGetLastError());
         launch_count_add(1);
     }
     if (P.totalRowGroups > 0) {
-        bf_flags_kernel<<<std::min<uint32_t>((P.totalRowGroups + 7) / 8, uint32_t(nsm) * 64u), 256, 0, stream>>>(P);
+        bf_flags_kernel<N><<<std::min<uint32_t>((P.totalRowGroups + 7) / 8, uint32_t(nsm) * 64u), 256, 0, stream>>>(P);
         RSFM_CUDA_TRY(cudaGetLastError());
         launch_count_add(1);
     }
@@ -783,7 +797,7 @@ static int launch_match(const Params& P, int nsm, cudaStream_t stream) {
 }
 
 // Fills a task's device description and counts it into P's totals. Empty sides get no units.
-static int fill_task(TaskDev* T, const rsfm_sift_bf_task& in, uint32_t* second, uint32_t* flags, Params* P) {
+static int fill_task(TaskDev* T, const rsfm_sift_bf_task& in, uint32_t* second, uint32_t* flags, ParamsBase* P) {
     T->nA = in.nbDescA;
     T->nB = in.nbDescB;
     T->descA = static_cast<const uint4*>(in.descA);
@@ -810,8 +824,9 @@ static int fill_task(TaskDev* T, const rsfm_sift_bf_task& in, uint32_t* second, 
     return RSFM_OK;
 }
 
-int launch_chunk(const rsfm_sift_bf_task* tasks, size_t n, uint32_t* const* second, uint32_t* const* flags,
-                 uint32_t ratioNum, uint32_t ratioDen, cudaStream_t stream, bool initialised) {
+template <int N>
+static int launch_tasks(const rsfm_sift_bf_task* tasks, size_t n, uint32_t* const* second, uint32_t* const* flags,
+                        uint32_t ratioNum, uint32_t ratioDen, cudaStream_t stream, bool initialised) {
     const int nsm = sm_count();
     if (nsm <= 0) return RSFM_ERR_CUDA;
 
@@ -829,8 +844,8 @@ int launch_chunk(const rsfm_sift_bf_task* tasks, size_t n, uint32_t* const* seco
         launch_count_add(1);
     }
 
-    Params P;
-    memset(&P, 0, sizeof(P));
+    Params<N> P;
+    memset(static_cast<void*>(&P), 0, sizeof(P));
     P.unitBlocks = choose_unit_blocks(sizes, nsm);
     P.ratioNum = ratioNum;
     P.ratioDen = ratioDen;
@@ -843,10 +858,16 @@ int launch_chunk(const rsfm_sift_bf_task* tasks, size_t n, uint32_t* const* seco
     if (!P.err) return RSFM_ERR_CUDA;
     if (P.totalUnits > 0 || P.totalRowGroups > 0) {
         P.fused = fuse_phases(P, nsm) ? 1u : 0u;
-        const int st = second ? launch_match<true>(P, nsm, stream) : launch_match<false>(P, nsm, stream);
+        const int st = second ? launch_match<true, N>(P, nsm, stream) : launch_match<false, N>(P, nsm, stream);
         if (st != RSFM_OK) return st;
     }
     return RSFM_OK;
+}
+
+int launch_chunk(const rsfm_sift_bf_task* tasks, size_t n, uint32_t* const* second, uint32_t* const* flags,
+                 uint32_t ratioNum, uint32_t ratioDen, cudaStream_t stream, bool initialised) {
+    return n == 1 ? launch_tasks<1>(tasks, n, second, flags, ratioNum, ratioDen, stream, initialised)
+                  : launch_tasks<kMaxTasksPerLaunch>(tasks, n, second, flags, ratioNum, ratioDen, stream, initialised);
 }
 
 // ---------------------------------------------------------------- batched plans
@@ -868,7 +889,7 @@ __global__ void plan_init_kernel(const TaskDev* __restrict__ tasks) {
 
 struct rsfm_bf_plan {
     rsfm_b200::bf::TaskDev* dTasks = nullptr;
-    rsfm_b200::bf::Params P;
+    rsfm_b200::bf::Params<1> P;
     uint32_t nTasks = 0;
     uint32_t blocksX = 1;
     int nsm = 0;
@@ -885,7 +906,7 @@ static int plan_enqueue(rsfm_bf_plan* pl, cudaStream_t s) {
     launch_count_add(1);
     plan_init_kernel<<<dim3(pl->blocksX, pl->nTasks), 256, 0, s>>>(pl->dTasks);
     RSFM_CUDA_TRY(cudaGetLastError());
-    return launch_match<true>(pl->P, pl->nsm, s);
+    return launch_match<true, 1>(pl->P, pl->nsm, s);
 }
 
 int validate(const rsfm_sift_bf_task* tasks, size_t n) {
@@ -962,7 +983,7 @@ extern "C" int rsfm_bf_plan_create(const rsfm_sift_bf_task* tasks, size_t nbTask
     const int nsm = sm_count();
     if (nsm <= 0) return RSFM_ERR_CUDA;
     auto* pl = new rsfm_bf_plan();
-    memset(&pl->P, 0, sizeof(pl->P));
+    memset(static_cast<void*>(&pl->P), 0, sizeof(pl->P));
     std::vector<std::pair<uint32_t, uint32_t>> sizes;
     uint32_t maxN = 1;
     for (size_t t = 0; t < nbTasks; ++t) {
@@ -1012,7 +1033,7 @@ extern "C" int rsfm_bf_plan_create(const rsfm_sift_bf_task* tasks, size_t nbTask
     const bool useGraph = !opts || opts->useGraph;
     if (useGraph) {
         // Set kernel attributes outside the capture, then record the launches once.
-        st = bf::ensure_attr<true>();
+        st = bf::ensure_attr<true, 1>();
         if (st != RSFM_OK) {
             rsfm_bf_plan_destroy(pl);
             return st;
