@@ -896,7 +896,7 @@ struct rsfm_bf_plan {
     cudaStream_t capture = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    uint32_t launches = 0;
+    uint32_t launches = 0;  // kernels in the graph
 };
 
 namespace rsfm_b200 {
@@ -1043,7 +1043,9 @@ extern "C" int rsfm_bf_plan_create(const rsfm_sift_bf_task* tasks, size_t nbTask
             rsfm_bf_plan_destroy(pl);
             return RSFM_ERR_CUDA;
         }
+        launch_count_reset();
         st = bf::plan_enqueue(pl, pl->capture);
+        pl->launches = rsfm_last_launch_count();
         cudaGraph_t g = nullptr;
         const cudaError_t e = cudaStreamEndCapture(pl->capture, &g);
         pl->graph = g;
@@ -1065,7 +1067,7 @@ extern "C" int rsfm_bf_plan_launch(rsfm_bf_plan* plan, cudaStream_t stream) {
         const bool prof = profile_begin(stream, &tok);
         RSFM_CUDA_TRY(cudaGraphLaunch(plan->exec, stream));
         if (prof) profile_end(stream, tok);
-        launch_count_add(plan->P.totalUnits > 0 ? 4 : 2);
+        launch_count_add(plan->launches);
     } else {
         const int st = bf::plan_enqueue(plan, stream);
         if (st != RSFM_OK) return st;

@@ -134,6 +134,21 @@ def test_plan_batched_workload_sizes(rsfm, oracle):
         plan.close()
 
 
+@pytest.mark.parametrize("sizes", [[(700, 900)], [(9000, 9100), (40, 300)], [(0, 50)], [(30, 0)], [(0, 0), (30, 40)]])
+def test_plan_launch_count(rsfm, sizes):
+    """A replayed graph reports the launches that it holds: as many as the plan without a graph makes."""
+    counts = []
+    for graph in (False, True):
+        tasks = [rsfm.BFTask(torch.zeros((na, 128), dtype=torch.uint8, device="cuda"),
+                             torch.ones((nb, 128), dtype=torch.uint8, device="cuda")) for na, nb in sizes]
+        plan = rsfm.BFPlan(tasks, use_graph=graph)
+        plan.launch()
+        counts.append(rsfm.last_launch_count())
+        torch.cuda.synchronize()
+        plan.close()
+    assert counts[0] == counts[1] > 0
+
+
 def test_device_generator_distribution(rsfm):
     g = torch.Generator(device="cuda")
     g.manual_seed(3)
