@@ -560,8 +560,9 @@ const char* rsfm_last_cuda_error(void);
 uint32_t rsfm_last_launch_count(void);
 
 /* Diagnostics (no reference counterpart). When enabled, every matcher call brackets its dominant
- * kernel with two CUDA events on the caller's stream; rsfm_profile_collect waits for them and
- * returns the summed kernel time (ms) and the number of bracketed launches, then resets. */
+ * kernel with two CUDA events on the caller's stream (brute force: matcher, index resolution and
+ * flags; a plan: its whole launch); rsfm_profile_collect waits for them and returns the summed
+ * time (ms) and the number of brackets, then resets. */
 int rsfm_profile_enable(int on);
 int rsfm_profile_collect(float* totalMs, uint32_t* launches);
 

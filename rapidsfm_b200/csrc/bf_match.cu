@@ -767,8 +767,6 @@ template <bool kSecond, int N>
 static int launch_match(const Params<N>& P, int nsm, cudaStream_t stream) {
     const int st = ensure_attr<kSecond, N>();
     if (st != RSFM_OK) return st;
-    void* tok = nullptr;
-    const bool prof = profile_begin(stream, &tok);
     if (P.fused) {
         // a CTA per unit, or enough for the results of a few units with many columns
         const uint32_t want = std::max(P.totalUnits, std::max(P.totalGroups, P.totalRowGroups) / (kThreads / 32) + 1);
@@ -780,7 +778,6 @@ static int launch_match(const Params<N>& P, int nsm, cudaStream_t stream) {
         bf_match_kernel<kSecond, N><<<std::min<uint32_t>(P.totalUnits, uint32_t(nsm)), kThreads, sizeof(Smem) + 1024, stream>>>(P);
         RSFM_CUDA_TRY(cudaGetLastError());
     }
-    if (prof) profile_end(stream, tok);
     launch_count_add(1);
     if (P.fused) return RSFM_OK;
     if (P.totalGroups > 0) {
@@ -858,8 +855,12 @@ static int launch_tasks(const rsfm_sift_bf_task* tasks, size_t n, uint32_t* cons
     if (!P.err) return RSFM_ERR_CUDA;
     if (P.totalUnits > 0 || P.totalRowGroups > 0) {
         P.fused = fuse_phases(P, nsm) ? 1u : 0u;
+        // the bracket of rsfm_profile_* holds all that produces the results, initialisation apart
+        void* tok = nullptr;
+        const bool prof = profile_begin(stream, &tok);
         const int st = second ? launch_match<true, N>(P, nsm, stream) : launch_match<false, N>(P, nsm, stream);
         if (st != RSFM_OK) return st;
+        if (prof) profile_end(stream, tok);
     }
     return RSFM_OK;
 }
@@ -1062,16 +1063,17 @@ extern "C" int rsfm_bf_plan_create(const rsfm_sift_bf_task* tasks, size_t nbTask
 extern "C" int rsfm_bf_plan_launch(rsfm_bf_plan* plan, cudaStream_t stream) {
     launch_count_reset();
     if (!plan) return RSFM_ERR_INVALID_ARG;
+    // (bracketed here and not in plan_enqueue: an event recorded while capturing cannot be read)
+    void* tok = nullptr;
+    const bool prof = profile_begin(stream, &tok);
     if (plan->exec) {
-        void* tok = nullptr;
-        const bool prof = profile_begin(stream, &tok);
         RSFM_CUDA_TRY(cudaGraphLaunch(plan->exec, stream));
-        if (prof) profile_end(stream, tok);
         launch_count_add(plan->launches);
     } else {
         const int st = bf::plan_enqueue(plan, stream);
         if (st != RSFM_OK) return st;
     }
+    if (prof) profile_end(stream, tok);
     return RSFM_OK;
 }
 

@@ -149,6 +149,58 @@ def test_plan_launch_count(rsfm, sizes):
     assert counts[0] == counts[1] > 0
 
 
+def test_plan_profile_brackets(rsfm):
+    """rsfm_profile_*: one bracket a launch of a plan, none left behind by the capture of its graph (an
+    event recorded while capturing cannot be read)."""
+    import ctypes
+    lib = rsfm._lib.load()
+    ms, n = ctypes.c_float(0), ctypes.c_uint32(0)
+
+    def collect():
+        rsfm._lib.check(lib.rsfm_profile_collect(ctypes.byref(ms), ctypes.byref(n)), "rsfm_profile_collect")
+        return n.value, ms.value
+
+    q, t, _ = synth.make_pair(700, 900, 0.5, 8.0, seed=3)
+    task = rsfm.BFTask(torch.from_numpy(q).cuda(), torch.from_numpy(t).cuda())
+    lib.rsfm_profile_enable(1)
+    try:
+        for graph in (False, True):
+            plan = rsfm.BFPlan([task], use_graph=graph)
+            plan.launch()
+            plan.launch()
+            launches, total = collect()
+            assert launches == 2 and total > 0
+            plan.close()
+    finally:
+        lib.rsfm_profile_enable(0)
+
+
+def test_profile_bracket_covers_the_results(rsfm):
+    """The bracket of a call holds every kernel that produces its results: what is outside of it at
+    32768 x 32768 is the initialisation (about 3 us with two event records; index resolution takes 15)."""
+    import ctypes
+    lib = rsfm._lib.load()
+    ms, n = ctypes.c_float(0), ctypes.c_uint32(0)
+    d = torch.randint(0, 100, (32768, 128), dtype=torch.uint8, device="cuda")
+    task = rsfm.BFTask(d, d.flip(0).contiguous())
+    rsfm.bf_match([task])
+    outside = []
+    lib.rsfm_profile_enable(1)
+    try:
+        for _ in range(12):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda._sleep(400000)  # the launches wait in the stream: no host time between them
+            e0.record()
+            rsfm.bf_match([task])
+            e1.record()
+            e1.synchronize()
+            rsfm._lib.check(lib.rsfm_profile_collect(ctypes.byref(ms), ctypes.byref(n)), "rsfm_profile_collect")
+            outside.append(1e3 * (e0.elapsed_time(e1) - ms.value))
+    finally:
+        lib.rsfm_profile_enable(0)
+    assert min(outside) < 9.0, outside
+
+
 def test_device_generator_distribution(rsfm):
     g = torch.Generator(device="cuda")
     g.manual_seed(3)
