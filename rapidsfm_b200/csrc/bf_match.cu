@@ -46,7 +46,6 @@
 #include "sm100.cuh"
 #include <algorithm>
 #include <climits>
-#include <cooperative_groups.h>
 #include <vector>
 
 namespace rsfm_b200 {
@@ -79,9 +78,8 @@ struct alignas(64) TaskDev {
     uint32_t* flagsA;   // null: no flags
     uint32_t nA, nB;
     uint32_t rowBlocks;
-    uint32_t unitBegin;   // first unit, first group of 4 results to resolve, first group of 32 rows:
-    uint32_t groupBegin;  // each in the order of the tasks
-    uint32_t rowGroupBegin;
+    uint32_t unitBegin;   // first unit and first group of 4 results to resolve, in the order of the
+    uint32_t groupBegin;  // tasks
 };
 
 // Launch parameters, with room for kTasks tasks: one (also for plans, whose tasks are in global memory)
@@ -91,9 +89,8 @@ struct ParamsBase {
     const TaskDev* gtasks;  // when non-null: any number of tasks, in global memory
     uint32_t nTasks;
     uint32_t totalUnits;
-    uint32_t totalGroups, totalRowGroups;  // totalRowGroups: 0 without flags
+    uint32_t totalGroups;
     uint32_t ratioNum, ratioDen;
-    uint32_t fused;       // cooperative launch: the matcher also resolves and sets the flags
     uint32_t unitBlocks;  // 256-column blocks per unit (<= 32: the chunk code holds 8 * 32 values)
     uint32_t* err;
 };
@@ -221,17 +218,18 @@ __device__ __forceinline__ void add_residuals(uint32_t (&x)[32], const int32_t* 
 
 // ---------------------------------------------------------------- index inside the winning chunk
 // The matcher leaves (distance, first index of a 16-descriptor chunk) per row and per column; eight
-// lanes per item compute the chunk's 16 exact distances (each lane 16 bytes of every descriptor:
-// one cache line per descriptor) and keep the first index at that distance. With `second`, the
-// chunk's other distances complete the second-best. Bound by L2 reads, 2 KiB per item: 134 MB for
+// lanes per result compute the chunk's 16 exact distances (each lane 16 bytes of every descriptor:
+// one cache line per descriptor) and keep the first index at that distance. A row's other distances
+// complete its second-best, and its flags follow. Bound by L2 reads, 2 KiB per result: 134 MB for
 // 32768 x 32768; chunks of 32 values would save the matcher 4 of 48 operations per 64 values and
 // double these reads.
-__device__ __forceinline__ void resolve_item(const uint4* __restrict__ q, const uint4* __restrict__ set, uint32_t nSet,
-                                             uint32_t normQ, const uint32_t* __restrict__ sqrSet,
-                                             unsigned long long* best, uint32_t* second, bool in, uint32_t l8) {
-    const unsigned long long bst = in ? __ldcg(best) : ~0ull;
-    const uint32_t j0 = uint32_t(bst), d = uint32_t(bst >> 32);
-    const bool has = in && j0 != ~0u;
+
+// Exact distances of q to the 16 descriptors of `set` from j0 on: lane l8 of the eight ends up with
+// candidates 2 * l8 and 2 * l8 + 1 (~0u past the end, or without `has`).
+__device__ __forceinline__ void chunk_distances(const uint4* __restrict__ q, uint32_t normQ,
+                                                const uint4* __restrict__ set, const uint32_t* __restrict__ sqrSet,
+                                                uint32_t nSet, uint32_t j0, bool has, uint32_t l8,
+                                                uint32_t (&dist)[2]) {
     uint32_t dot[kChunk];
     uint4 qv = make_uint4(0, 0, 0, 0), tv[kChunk];
     if (has) qv = __ldg(&q[l8]);
@@ -240,7 +238,6 @@ __device__ __forceinline__ void resolve_item(const uint4* __restrict__ q, const 
         tv[k] = make_uint4(0, 0, 0, 0);
         if (has && j0 + k < nSet) tv[k] = __ldg(&set[size_t(j0 + k) * 8 + l8]);
     }
-    // this lane ends up with the sums of candidates 2 * l8 and 2 * l8 + 1
     uint32_t nv[2] = {0, 0};
 #pragma unroll
     for (uint32_t e = 0; e < 2; ++e)
@@ -262,78 +259,92 @@ __device__ __forceinline__ void resolve_item(const uint4* __restrict__ q, const 
             dot[k] = mine + __shfl_xor_sync(0xffffffffu, theirs, o);
         }
     }
-    uint32_t dist[2], at = ~0u;
 #pragma unroll
-    for (int e = 1; e >= 0; --e) {
-        const uint32_t j = j0 + 2 * l8 + e;
-        dist[e] = has && j < nSet ? normQ + nv[e] - 2u * dot[e] : ~0u;
-        if (has && j < nSet && dist[e] == d) at = j;
-    }
-#pragma unroll
-    for (uint32_t o = 1; o < 8; o <<= 1) at = min(at, __shfl_xor_sync(0xffffffffu, at, o));
-    uint32_t s = ~0u;  // (shuffled by every lane: rows and columns may share a warp)
-#pragma unroll
-    for (int e = 0; e < 2; ++e)
-        if (j0 + 2 * l8 + e != at) s = min(s, dist[e]);
-#pragma unroll
-    for (uint32_t o = 1; o < 8; o <<= 1) s = min(s, __shfl_xor_sync(0xffffffffu, s, o));
-    if (second && has && l8 == 0 && s < __ldcg(second)) *second = s;
-    if (has && l8 == 0 && at != ~0u) *best = (static_cast<unsigned long long>(d) << 32) | at;
+    for (uint32_t e = 0; e < 2; ++e) dist[e] = has && j0 + 2 * l8 + e < nSet ? normQ + nv[e] - 2u * dot[e] : ~0u;
 }
 
-// Last task at or after t whose `begin` is <= w (tasks without any share their successor's).
+// Last task whose groups begin at or before w (tasks without any share their successor's).
 template <int N>
-__device__ __forceinline__ uint32_t task_at(const Params<N>& P, uint32_t t, uint32_t TaskDev::*begin, uint32_t w) {
-    uint32_t hi = P.nTasks - 1u;
+__device__ __forceinline__ uint32_t task_at(const Params<N>& P, uint32_t w) {
+    uint32_t t = 0, hi = P.nTasks - 1u;
     while (t < hi) {
         const uint32_t mid = (t + hi + 1u) >> 1;
-        if (task_of(P, mid).*begin <= w) t = mid; else hi = mid - 1u;
+        if (task_of(P, mid).groupBegin <= w) t = mid; else hi = mid - 1u;
     }
     return t;
 }
 
-// Warp w0 of `warps` takes a run of consecutive groups of four results (rows of A, then columns of
-// B), eight lanes a result.
+// Every warp takes a run of consecutive groups of four results (columns of B, then rows of A, so that
+// most columns are final when a row looks its match's up), eight lanes a result.
+//
+// A row's cross-check bit needs the final index of its match's column, which another warp may not have
+// written yet. It is decided from either state: the column's distance must be the row's; then its
+// index is the row itself (also as a chunk's first index: no earlier row of that chunk), or another
+// row, or the first index of the row's own chunk - and in that last case the row is the column's match
+// exactly if no earlier row of the chunk is as close. The alternatives: a grid-wide barrier (one
+// cooperative launch for matching, resolution and flags) needs all its blocks resident at once, which
+// a green context or a long kernel on another stream does not give (600 x 600, one call alone with all
+// outputs: 74 us, against 68 this way); a launch of its own for the flags costs 2 us in small
+// calls and re-reads the results in large ones (16384 x 16384 94 us against 90).
 template <int N>
-__device__ __forceinline__ void resolve_phase(const Params<N>& P, uint32_t w0, uint32_t warps, uint32_t lane) {
-    const uint32_t l8 = lane & 7u;
-    uint32_t t = 0;
-    const uint32_t run = (P.totalGroups + warps - 1u) / warps, first = w0 * run;
-    const uint32_t end = first < P.totalGroups ? min(P.totalGroups, first + run) : first;
-    if (first < end) t = task_at(P, 0u, &TaskDev::groupBegin, first);
+__global__ void __launch_bounds__(256) bf_resolve_kernel(const __grid_constant__ Params<N> P) {
+    const uint32_t lane = threadIdx.x & 31u, l8 = lane & 7u;
+    const uint32_t warps = gridDim.x * 8u;
+    const uint32_t run = (P.totalGroups + warps - 1u) / warps;
+    const uint32_t first = (blockIdx.x * 8u + (threadIdx.x >> 5)) * run;
+    if (first >= P.totalGroups) return;
+    const uint32_t end = min(P.totalGroups, first + run);
+    uint32_t t = task_at(P, first);
     for (uint32_t w = first; w < end; ++w) {
         while (t + 1 < P.nTasks && task_of(P, t + 1).groupBegin <= w) ++t;
         const TaskDev& T = task_of(P, t);
         const uint64_t x = uint64_t(w - T.groupBegin) * 4u + (lane >> 3);
-        const bool row = x < T.nA, in = x < uint64_t(T.nA) + T.nB;
-        const uint32_t i = row ? uint32_t(x) : in ? uint32_t(x - T.nA) : 0u;
-        const uint4* q = (row ? T.descA : T.descB) + size_t(i) * 8;
-        const uint32_t nq = in ? __ldg((row ? T.sqrA : T.sqrB) + i) : 0u;
-        resolve_item(q, row ? T.descB : T.descA, row ? T.nB : T.nA, nq, row ? T.sqrB : T.sqrA,
-                     (row ? T.bestA : T.bestB) + i, row && T.secondA ? T.secondA + i : nullptr, in, l8);
-    }
-}
-
-// Flags of every row: bit0 ratio test, bit1 cross-check. Runs of 32-row groups as above.
-template <int N>
-__device__ __forceinline__ void flags_phase(const Params<N>& P, uint32_t w0, uint32_t warps, uint32_t lane) {
-    uint32_t t = 0;
-    const uint32_t run = (P.totalRowGroups + warps - 1u) / warps, first = w0 * run;
-    const uint32_t end = first < P.totalRowGroups ? min(P.totalRowGroups, first + run) : first;
-    if (first < end) t = task_at(P, 0u, &TaskDev::rowGroupBegin, first);
-    for (uint32_t w = first; w < end; ++w) {
-        while (t + 1 < P.nTasks && task_of(P, t + 1).rowGroupBegin <= w) ++t;
-        const TaskDev& T = task_of(P, t);
-        const uint32_t i = (w - T.rowGroupBegin) * 32u + lane;
-        if (i >= T.nA) continue;
-        const unsigned long long bm = __ldcg(&T.bestA[i]);
-        const uint32_t j = uint32_t(bm & 0xFFFFFFFFu), d = uint32_t(bm >> 32);
-        uint32_t f = 0;
-        if (j != ~0u) {
-            if (uint64_t(P.ratioDen) * d < uint64_t(P.ratioNum) * __ldcg(&T.secondA[i])) f |= 1u;
-            if (j < T.nB && uint32_t(__ldcg(&T.bestB[j]) & 0xFFFFFFFFu) == i) f |= 2u;
+        const bool col = x < T.nB, row = !col && x < uint64_t(T.nA) + T.nB;
+        const uint32_t i = col ? uint32_t(x) : row ? uint32_t(x - T.nB) : 0u;
+        unsigned long long* best = (col ? T.bestB : T.bestA) + i;
+        const unsigned long long bst = col || row ? __ldcg(best) : ~0ull;
+        const uint32_t j0 = uint32_t(bst), d = uint32_t(bst >> 32);
+        const bool has = j0 != ~0u;
+        uint32_t dist[2];
+        chunk_distances((col ? T.descB : T.descA) + size_t(i) * 8, has ? __ldg((col ? T.sqrB : T.sqrA) + i) : 0u,
+                        col ? T.descA : T.descB, col ? T.sqrA : T.sqrB, col ? T.nA : T.nB, j0, has, l8, dist);
+        uint32_t at = ~0u, s = ~0u;
+#pragma unroll
+        for (int e = 1; e >= 0; --e)
+            if (has && dist[e] == d && dist[e] != ~0u) at = j0 + 2 * l8 + e;
+#pragma unroll
+        for (uint32_t o = 1; o < 8; o <<= 1) at = min(at, __shfl_xor_sync(0xffffffffu, at, o));
+        if (has && l8 == 0 && at != ~0u) __stcg(best, (static_cast<unsigned long long>(d) << 32) | at);
+        if (!__any_sync(0xffffffffu, row && T.secondA)) continue;
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+            if (j0 + 2 * l8 + e != at) s = min(s, dist[e]);
+#pragma unroll
+        for (uint32_t o = 1; o < 8; o <<= 1) s = min(s, __shfl_xor_sync(0xffffffffu, s, o));
+        if (row && l8 == 0) {
+            const uint32_t old = __ldcg(&T.secondA[i]);
+            if (s < old) T.secondA[i] = s;
+            s = min(s, old);
         }
-        T.flagsA[i] = f;
+        if (!T.flagsA) continue;
+        const uint32_t j = at != ~0u ? at : j0, c0 = i & ~(kChunk - 1u);
+        unsigned long long cb = row && j < T.nB ? __ldcg(&T.bestB[j]) : ~0ull;
+        cb = __shfl_sync(0xffffffffu, cb, int(lane & 24u));  // one state of it for the eight lanes
+        const bool near = row && has && uint32_t(cb >> 32) == d;
+        bool mutual = near && uint32_t(cb) == i;
+        const bool open = near && !mutual && uint32_t(cb) == c0;
+        if (__any_sync(0xffffffffu, open)) {
+            chunk_distances(T.descB + size_t(open ? j : 0u) * 8, open ? __ldg(&T.sqrB[j]) : 0u, T.descA, T.sqrA, T.nA, c0,
+                            open, l8, dist);
+            const bool closer = (c0 + 2 * l8 < i && dist[0] == d) || (c0 + 2 * l8 + 1 < i && dist[1] == d);
+            const uint32_t any = __ballot_sync(0xffffffffu, open && closer);
+            if (open) mutual = ((any >> (lane & 24u)) & 0xFFu) == 0u;
+        }
+        if (row && l8 == 0) {
+            uint32_t f = mutual ? 2u : 0u;
+            if (has && uint64_t(P.ratioDen) * d < uint64_t(P.ratioNum) * s) f |= 1u;
+            T.flagsA[i] = f;
+        }
     }
 }
 
@@ -666,29 +677,6 @@ __global__ void __launch_bounds__(kThreads, 1) bf_match_kernel(const __grid_cons
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, 512);
-    __syncwarp();
-
-    if (!P.fused) return;
-    // ---- every unit of the launch is published: indexes inside the winning chunks, then the flags,
-    // as phases of one cooperative launch (all CTAs are resident, and every wait above ends)
-    const cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-    grid.sync();
-    const uint32_t warps = gridDim.x * (kThreads / 32u), w0 = blockIdx.x * (kThreads / 32u) + warp;
-    resolve_phase(P, w0, warps, lane);
-    if (kSecond && P.totalRowGroups > 0) {
-        grid.sync();
-        flags_phase(P, w0, warps, lane);
-    }
-}
-
-// The same two phases as launches of their own.
-template <int N>
-__global__ void __launch_bounds__(256) bf_resolve_kernel(const __grid_constant__ Params<N> P) {
-    resolve_phase(P, blockIdx.x * 8u + (threadIdx.x >> 5), gridDim.x * 8u, threadIdx.x & 31u);
-}
-template <int N>
-__global__ void __launch_bounds__(256) bf_flags_kernel(const __grid_constant__ Params<N> P) {
-    flags_phase(P, blockIdx.x * 8u + (threadIdx.x >> 5), gridDim.x * 8u, threadIdx.x & 31u);
 }
 
 // Initialise results: bestA/bestB = {~0u, ~0u}, secondA = ~0u.
@@ -754,46 +742,26 @@ static int ensure_attr() {
     return set_max_dynamic_smem(reinterpret_cast<const void*>(bf_match_kernel<kSecond, N>), sizeof(Smem) + 1024);
 }
 
-// Up to eight blocks per SM, and results for one round of the resolving warps, a call is bound by its
-// host time (2 us and more a launch), so matching, index resolution and flags share one launch;
-// beyond, the grid-wide barriers between them cost more than launches (one launch against three, us
-// a call with all outputs: 4096 x 4096 47 and 57, 8192 x 8192 53.5 and 55, 10000 x 10000 68 and 56.5).
-static bool fuse_phases(const ParamsBase& P, int nsm) {
-    return uint64_t(P.totalUnits) * P.unitBlocks <= uint64_t(nsm) * 8 && P.totalGroups <= uint32_t(nsm) * 28u;
-}
-
 // The matcher and what follows it.
 template <bool kSecond, int N>
 static int launch_match(const Params<N>& P, int nsm, cudaStream_t stream) {
-    const int st = ensure_attr<kSecond, N>();
-    if (st != RSFM_OK) return st;
-    if (P.fused) {
-        // a CTA per unit, or enough for the results of a few units with many columns
-        const uint32_t want = std::max(P.totalUnits, std::max(P.totalGroups, P.totalRowGroups) / (kThreads / 32) + 1);
-        void* args[] = {const_cast<Params<N>*>(&P)};
-        RSFM_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(bf_match_kernel<kSecond, N>),
-                                                  dim3(std::min<uint32_t>(want, uint32_t(nsm))), dim3(kThreads), args,
-                                                  sizeof(Smem) + 1024, stream));
-    } else if (P.totalUnits > 0) {
+    if (P.totalUnits > 0) {
+        const int st = ensure_attr<kSecond, N>();
+        if (st != RSFM_OK) return st;
         bf_match_kernel<kSecond, N><<<std::min<uint32_t>(P.totalUnits, uint32_t(nsm)), kThreads, sizeof(Smem) + 1024, stream>>>(P);
-        RSFM_CUDA_TRY(cudaGetLastError());
-    }
-    launch_count_add(1);
-    if (P.fused) return RSFM_OK;
-    if (P.totalGroups > 0) {
-        bf_resolve_kernel<N><<<std::min<uint32_t>((P.totalGroups + 7) / 8, uint32_t(nsm) * 64u), 256, 0, stream>>>(P);
         RSFM_CUDA_TRY(cudaGetLastError());
         launch_count_add(1);
     }
-    if (P.totalRowGroups > 0) {
-        bf_flags_kernel<N><<<std::min<uint32_t>((P.totalRowGroups + 7) / 8, uint32_t(nsm) * 64u), 256, 0, stream>>>(P);
+    if (P.totalGroups > 0) {
+        bf_resolve_kernel<N><<<std::min<uint32_t>((P.totalGroups + 7) / 8, uint32_t(nsm) * 64u), 256, 0, stream>>>(P);
         RSFM_CUDA_TRY(cudaGetLastError());
         launch_count_add(1);
     }
     return RSFM_OK;
 }
 
-// Fills a task's device description and counts it into P's totals. Empty sides get no units.
+// Fills a task's device description and counts it into P's totals. Empty sides get no units, and of
+// the results only rows with flags need a look.
 static int fill_task(TaskDev* T, const rsfm_sift_bf_task& in, uint32_t* second, uint32_t* flags, ParamsBase* P) {
     T->nA = in.nbDescA;
     T->nB = in.nbDescB;
@@ -807,9 +775,8 @@ static int fill_task(TaskDev* T, const rsfm_sift_bf_task& in, uint32_t* second, 
     T->flagsA = flags;
     T->unitBegin = P->totalUnits;
     T->groupBegin = P->totalGroups;
-    T->rowGroupBegin = P->totalRowGroups;
     T->rowBlocks = 1;
-    if (flags) P->totalRowGroups += (T->nA + 31) / 32;
+    if (T->nA > 0 && (T->nB > 0 || flags)) P->totalGroups += uint32_t((uint64_t(T->nA) + T->nB + 3) / 4);
     if (T->nA == 0 || T->nB == 0) return RSFM_OK;
     int st = encode_desc_tmap(&T->tmA, in.descA, T->nA, kUnitRows);
     if (st == RSFM_OK) st = encode_desc_tmap(&T->tmB, in.descB, T->nB, kBlockCols);
@@ -817,7 +784,6 @@ static int fill_task(TaskDev* T, const rsfm_sift_bf_task& in, uint32_t* second, 
     T->rowBlocks = (T->nA + kUnitRows - 1) / kUnitRows;
     const uint32_t unitCols = kBlockCols * P->unitBlocks;
     P->totalUnits += T->rowBlocks * ((T->nB + unitCols - 1) / unitCols);
-    P->totalGroups += uint32_t((uint64_t(T->nA) + T->nB + 3) / 4);
     return RSFM_OK;
 }
 
@@ -853,8 +819,7 @@ static int launch_tasks(const rsfm_sift_bf_task* tasks, size_t n, uint32_t* cons
     P.nTasks = uint32_t(n);
     P.err = device_error_word();
     if (!P.err) return RSFM_ERR_CUDA;
-    if (P.totalUnits > 0 || P.totalRowGroups > 0) {
-        P.fused = fuse_phases(P, nsm) ? 1u : 0u;
+    if (P.totalUnits > 0 || P.totalGroups > 0) {
         // the bracket of rsfm_profile_* holds all that produces the results, initialisation apart
         void* tok = nullptr;
         const bool prof = profile_begin(stream, &tok);

@@ -16,8 +16,10 @@
 //   matcher widens each image once per call to one value (0..15) per byte in scratch, in the
 //   original dimension order, and runs the 8-bit kernel on it: the distance is a sum over
 //   dimensions, identical to the reference's u4 MMA distance.
+#include "bf_internal.h"
 #include "common.h"
 
+#include <algorithm>
 #include <map>
 #include <utility>
 #include <vector>
@@ -39,9 +41,15 @@ __global__ void pack_4b_kernel(uint2* __restrict__ dst, const uint4* __restrict_
 
 // One thread per 16 packed bytes (two groups), 32 widened bytes out in source order: the low
 // nibbles of packed word w are dimensions 8i..8i+3 of its group, the high nibbles 8i+4..8i+7.
-__global__ void widen_4b_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src, uint64_t chunks) {
-    for (uint64_t c = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; c < chunks;
-         c += uint64_t(gridDim.x) * blockDim.x) {
+// Also sets the results of nInit tasks to ~0, so that their match needs no launch for that.
+__global__ void widen_4b_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src, uint64_t chunks,
+                                const __grid_constant__ bf::InitParams I, uint32_t nInit) {
+    const uint64_t first = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x, step = uint64_t(gridDim.x) * blockDim.x;
+    for (uint32_t t = 0; t < nInit; ++t) {
+        for (uint64_t x = first; x < I.nA[t]; x += step) I.bestA[t][x] = ~0ull;
+        for (uint64_t x = first; x < I.nB[t]; x += step) I.bestB[t][x] = ~0ull;
+    }
+    for (uint64_t c = first; c < chunks; c += step) {
         const uint4 s = __ldg(&src[c]);
         dst[2 * c] = make_uint4(s.x & 0x0F0F0F0Fu, (s.x >> 4) & 0x0F0F0F0Fu, s.y & 0x0F0F0F0Fu,
                                 (s.y >> 4) & 0x0F0F0F0Fu);
@@ -207,17 +215,22 @@ extern "C" int rsfm_bf_match_4b(const rsfm_sift_bf_task* tasks, size_t nbTasks, 
         wide = static_cast<uint8_t*>(bfv::pool_alloc(im.total * 128, stream, &st));
         if (!wide) return st;
     }
+    // Widening image k also initialises the results of the k-th matcher launch (kMaxTasksPerLaunch tasks).
     uint32_t launches = 0;
+    size_t ready = 0;  // tasks whose results are initialised
     for (const auto& kv : im.offset) {
         const uint64_t chunks = uint64_t(kv.first.second) * 4;  // 16-byte chunks of 64-byte descriptors
+        const size_t n = std::min<size_t>(bf::kMaxTasksPerLaunch, nbTasks - ready);
         bfv::widen_4b_kernel<<<bfv::grid_for(chunks, 256), 256, 0, stream>>>(
-            reinterpret_cast<uint4*>(wide + kv.second * 128), static_cast<const uint4*>(kv.first.first), chunks);
+            reinterpret_cast<uint4*>(wide + kv.second * 128), static_cast<const uint4*>(kv.first.first), chunks,
+            bf::init_params(tasks + ready, n, nullptr), uint32_t(n));
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) {
             set_last_cuda_error(e, "widen_4b_kernel");
             st = RSFM_ERR_CUDA;
             break;
         }
+        ready += n;
         ++launches;
     }
     std::vector<rsfm_sift_bf_task> local(tasks, tasks + nbTasks);
@@ -225,12 +238,15 @@ extern "C" int rsfm_bf_match_4b(const rsfm_sift_bf_task* tasks, size_t nbTasks, 
         T.descA = T.nbDescA ? wide + 128 * im.offset.at({T.descA, T.nbDescA}) : nullptr;
         T.descB = T.nbDescB ? wide + 128 * im.offset.at({T.descB, T.nbDescB}) : nullptr;
     }
-    if (st == RSFM_OK) st = bfv::match_8b(local, stream, &launches);
+    launch_count_reset();
+    launch_count_add(launches);
+    for (size_t i = 0; i < nbTasks && st == RSFM_OK; i += bf::kMaxTasksPerLaunch) {
+        const size_t n = std::min<size_t>(bf::kMaxTasksPerLaunch, nbTasks - i);
+        st = bf::launch_chunk(local.data() + i, n, nullptr, nullptr, 0, 1, stream, i < ready);
+    }
     if (wide) {
         const cudaError_t e = cudaFreeAsync(wide, stream);
         if (st == RSFM_OK && e != cudaSuccess) st = RSFM_ERR_CUDA;
     }
-    launch_count_reset();
-    launch_count_add(launches);
     return st;
 }

@@ -169,15 +169,15 @@ def test_unit_and_chunk_edges(rsfm, oracle, na, nb, seed):
 
 @pytest.mark.parametrize("sizes", [[(700, 900), (300, 0), (0, 40), (1000, 20)], [(9000, 9100), (30, 8000)]])
 def test_phases_in_one_launch_and_apart(rsfm, oracle, sizes):
-    # Up to eight 256 x 256 blocks per SM a call is init + one cooperative launch; above, index
-    # resolution and flags are launches of their own. Same results, both entry points, empty sides.
+    # A call is init, match and resolution with flags, whatever its size. Same results from both entry
+    # points, empty sides.
     pairs = []
     for k, (na, nb) in enumerate(sizes):
         q, t, _ = synth.make_pair(max(na, 1), max(nb, 1), 0.5, 8.0, seed=500 + k)
         pairs.append((q[:na], t[:nb]))
     tasks = [rsfm.BFTask(_dev(a), _dev(b)) for a, b in pairs]
     rsfm.bf_match_ext(tasks)
-    assert rsfm.last_launch_count() == (2 if len(sizes) == 4 else 4)
+    assert rsfm.last_launch_count() == 3
     got = _run_ext(rsfm, pairs)
     rsfm.bf_match(tasks)
     for (a, b), g, t in zip(pairs, got, tasks):
@@ -211,3 +211,64 @@ def test_user_graph_capture_and_streams(rsfm, oracle):
         got = (np.stack(rsfm.unpack_best(t.bestA), 1), np.stack(rsfm.unpack_best(t.bestB), 1),
                t.secondA.cpu().numpy().view(np.uint32), t.flagsA.cpu().numpy().view(np.uint32))
         _check(oracle, a, b, got)
+
+
+@pytest.mark.parametrize("na,nb", [(64, 20000), (20000, 64), (1, 5000), (5000, 1)])
+def test_few_blocks_many_results(rsfm, oracle, na, nb):
+    # Long thin pairs: little matching, many results, and no launch more than a square pair's.
+    a, b = synth.make_pair(na, nb, 0.5, 8.0, seed=na + 2 * nb)[:2]
+    task = rsfm.BFTask(_dev(a), _dev(b))
+    rsfm.bf_match_ext([task])
+    assert rsfm.last_launch_count() == 3
+    _check(oracle, a, b, _run_ext(rsfm, [(a, b)])[0])
+
+
+@pytest.mark.parametrize("na,nb,seed", [(200, 150, 0), (3000, 2500, 1), (20000, 9000, 2)])
+def test_cross_check_among_equal_rows_of_a_chunk(rsfm, oracle, na, nb, seed):
+    """Runs of equal rows (1 to 24 long, so inside a 16-row chunk and across its edges): of the rows that
+    are as close to a column only the first is its match. Columns whose index is resolved before or after
+    the row that looks it up give the same flags, call after call."""
+    rng = np.random.default_rng(seed)
+    base = synth.make_pair(na, 1, 0.0, 1.0, seed=seed)[0]
+    a = np.repeat(base, rng.integers(1, 25, na), axis=0)[:na]
+    b = np.minimum(a[rng.integers(0, na, nb)] + (rng.random((nb, 128)) < 0.05 * rng.integers(0, 2, (nb, 1))), 255)
+    b = b.astype(np.uint8)
+    efwd, ebwd, esec = oracle.bf_match(a, b)
+    eflags = oracle.match_flags(efwd, esec, ebwd)
+    assert 0 < (eflags & 2).sum() < 2 * na
+    for _ in range(3):
+        fwd, bwd, sec, flags = _run_ext(rsfm, [(a, b)])[0]
+        np.testing.assert_array_equal(fwd, efwd)
+        np.testing.assert_array_equal(bwd, ebwd)
+        np.testing.assert_array_equal(sec, esec)
+        np.testing.assert_array_equal(flags, eflags)
+
+
+def test_stream_of_a_green_context(rsfm, oracle):
+    """A stream that owns 16 SMs: a call may not need all its blocks resident at once."""
+    cu = pytest.importorskip("cuda.bindings.driver")
+
+    def ok(r):
+        assert r[0] == cu.CUresult.CUDA_SUCCESS, r[0]
+        return r[1] if len(r) == 2 else r[1:]
+
+    torch.cuda.synchronize()  # (the primary context is there and current)
+    dev = ok(cu.cuDeviceGet(torch.cuda.current_device()))
+    sms = ok(cu.cuDeviceGetDevResource(dev, cu.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+    groups, _, _ = ok(cu.cuDevSmResourceSplitByCount(1, sms, 0, 16))
+    desc = ok(cu.cuDevResourceGenerateDesc(groups[:1], 1))
+    green = ok(cu.cuGreenCtxCreate(desc, dev, cu.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM))
+    raw = ok(cu.cuGreenCtxStreamCreate(green, cu.CUstream_flags.CU_STREAM_NON_BLOCKING, 0))
+    try:
+        stream = torch.cuda.ExternalStream(int(raw))
+        a, b = synth.make_pair(3000, 2500, 0.5, 8.0, seed=77)[:2]
+        task = rsfm.BFTask(_dev(a), _dev(b))
+        torch.cuda.synchronize()
+        rsfm.bf_match_ext([task], stream=stream)
+        stream.synchronize()
+        got = (np.stack(rsfm.unpack_best(task.bestA), 1), np.stack(rsfm.unpack_best(task.bestB), 1),
+               task.secondA.cpu().numpy().view(np.uint32), task.flagsA.cpu().numpy().view(np.uint32))
+        _check(oracle, a, b, got)
+    finally:
+        ok(cu.cuStreamDestroy(raw))
+        ok(cu.cuGreenCtxDestroy(green))

@@ -71,6 +71,30 @@ def test_bf_match_4b_shared_train(rsfm, oracle):
         np.testing.assert_array_equal(bwd, ebwd)
 
 
+@pytest.mark.parametrize("images,count", [(2, 40), (5, 33), (40, 17)])
+def test_bf_match_4b_results_initialised(rsfm, oracle, images, count):
+    # Widening image k initialises the results of tasks 16 k to 16 k + 15; with fewer images than that
+    # takes the matcher launches initialise the rest. Empty sides included.
+    im = [rsfm.sift_desc_8b_to_4b(_dev(synth.uniform_bytes(40 + 37 * k, 60 + k))) for k in range(images - 1)]
+    im.append(torch.empty((0, 64), dtype=torch.uint8, device="cuda"))
+    tasks = [rsfm.BFTask(im[k % images], im[(k // 2) % images], bits=4) for k in range(count)]
+    for t in tasks:
+        t.bestA.fill_(5)
+        t.bestB.fill_(7)
+    rsfm.bf_match_4b(tasks)
+    torch.cuda.synchronize()
+    values = [oracle.desc_4b_values(x.cpu().numpy()) if len(x) else None for x in im]
+    for k, t in enumerate(tasks):
+        fwd, bwd = _best(rsfm, t)
+        a, b = values[k % images], values[(k // 2) % images]
+        if a is None or b is None:
+            assert (fwd == 0xFFFFFFFF).all() and (bwd == 0xFFFFFFFF).all()
+            continue
+        efwd, ebwd, _ = oracle.bf_match(a, b)
+        np.testing.assert_array_equal(fwd, efwd)
+        np.testing.assert_array_equal(bwd, ebwd)
+
+
 def test_bf_match_idp_without_norms(rsfm, oracle):
     pairs = [synth.make_pair(2000, 2300, 0.6, 8.0, seed=31)[:2], synth.make_pair(400, 3000, 0.5, 10.0, seed=32)[:2]]
     tasks = [rsfm.BFTask(_dev(a), _dev(b), norms=False) for a, b in pairs]
