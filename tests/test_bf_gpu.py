@@ -272,3 +272,40 @@ def test_stream_of_a_green_context(rsfm, oracle):
     finally:
         ok(cu.cuStreamDestroy(raw))
         ok(cu.cuGreenCtxDestroy(green))
+
+
+def test_calls_whose_kernels_overlap(rsfm, oracle):
+    """A call's kernels start while the one before them runs. Calls one after the other without a wait,
+    on inputs written by a kernel just before each and into the same buffers, in all three forms (norms
+    and 4-bit widening right before the match): every result as if the call were alone."""
+    n = [(300, 900), (900, 300), (2300, 1200), (40, 5000)]
+    pairs = [[synth.make_pair(na, nb, 0.5, 8.0, seed=800 + 10 * k + r)[:2] for r in range(3)] for k, (na, nb) in enumerate(n)]
+    src = [[(_dev(a), _dev(b)) for a, b in p] for p in pairs]
+    bufs = [(torch.empty_like(p[0][0]), torch.empty_like(p[0][1])) for p in src]
+    got = []
+    for rep in range(4):
+        for k, (a, b) in enumerate(bufs):
+            for r in range(3):
+                a.copy_(src[k][r][0])
+                b.copy_(src[k][r][1])
+                ext, idp = rsfm.BFTask(a, b), rsfm.BFTask(a, b, norms=False)
+                rsfm.bf_match_ext([ext])
+                rsfm.bf_match_idp([idp])
+                four = rsfm.BFTask(rsfm.sift_desc_8b_to_4b(a), rsfm.sift_desc_8b_to_4b(b), bits=4)
+                rsfm.bf_match_4b([four])
+                got.append((k, r, ext, idp, four))
+    torch.cuda.synchronize()
+    assert rsfm.device_error() == 0
+    want = {}
+    for k, r, ext, idp, four in got:
+        a, b = pairs[k][r]
+        if (k, r) not in want:
+            fwd, bwd, sec = oracle.bf_match(a, b)
+            want[k, r] = (fwd, bwd, sec, oracle.match_flags(fwd, sec, bwd), oracle.bf_match(
+                oracle.desc_4b_values(oracle.desc_8b_to_4b(a)), oracle.desc_4b_values(oracle.desc_8b_to_4b(b))))
+        fwd, bwd, sec, flags, w4 = want[k, r]
+        for t, (f, g) in ((ext, (fwd, bwd)), (idp, (fwd, bwd)), (four, w4[:2])):
+            np.testing.assert_array_equal(np.stack(rsfm.unpack_best(t.bestA), 1), f)
+            np.testing.assert_array_equal(np.stack(rsfm.unpack_best(t.bestB), 1), g)
+        np.testing.assert_array_equal(ext.secondA.cpu().numpy().view(np.uint32), sec)
+        np.testing.assert_array_equal(ext.flagsA.cpu().numpy().view(np.uint32), flags)
