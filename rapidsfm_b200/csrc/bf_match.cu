@@ -78,8 +78,9 @@ struct alignas(64) TaskDev {
     uint32_t* flagsA;   // null: no flags
     uint32_t nA, nB;
     uint32_t rowBlocks;
-    uint32_t unitBegin;   // first unit and first group of 4 results to resolve, in the order of the
-    uint32_t groupBegin;  // tasks
+    uint32_t unitBegin;   // first unit, first group of 4 results to resolve, first group of 32 rows:
+    uint32_t groupBegin;  // each in the order of the tasks
+    uint32_t rowGroupBegin;
 };
 
 // Launch parameters, with room for kTasks tasks: one (also for plans, whose tasks are in global memory)
@@ -89,7 +90,7 @@ struct ParamsBase {
     const TaskDev* gtasks;  // when non-null: any number of tasks, in global memory
     uint32_t nTasks;
     uint32_t totalUnits;
-    uint32_t totalGroups;
+    uint32_t totalGroups, totalRowGroups;  // totalRowGroups: 0 without flags
     uint32_t ratioNum, ratioDen;
     uint32_t unitBlocks;  // 256-column blocks per unit (<= 32: the chunk code holds 8 * 32 values)
     uint32_t* err;
@@ -227,7 +228,7 @@ __device__ __forceinline__ void add_residuals(uint32_t (&x)[32], const int32_t* 
 // The matcher leaves (distance, first index of a 16-descriptor chunk) per row and per column; eight
 // lanes per result compute the chunk's 16 exact distances (each lane 16 bytes of every descriptor:
 // one cache line per descriptor) and keep the first index at that distance. A row's other distances
-// complete its second-best, and its flags follow. Bound by L2 reads, 2 KiB per result: 134 MB for
+// complete its second-best. Bound by L2 reads, 2 KiB per result: 134 MB for
 // 32768 x 32768; chunks of 32 values would save the matcher 4 of 48 operations per 64 values and
 // double these reads.
 
@@ -270,30 +271,30 @@ __device__ __forceinline__ void chunk_distances(const uint4* __restrict__ q, uin
     for (uint32_t e = 0; e < 2; ++e) dist[e] = has && j0 + 2 * l8 + e < nSet ? normQ + nv[e] - 2u * dot[e] : ~0u;
 }
 
-// Last task whose groups begin at or before w (tasks without any share their successor's).
+// Last task whose `begin` is at or before w (tasks without any share their successor's).
 template <int N>
-__device__ __forceinline__ uint32_t task_at(const Params<N>& P, uint32_t w) {
+__device__ __forceinline__ uint32_t task_at(const Params<N>& P, uint32_t TaskDev::*begin, uint32_t w) {
     uint32_t t = 0, hi = P.nTasks - 1u;
     while (t < hi) {
         const uint32_t mid = (t + hi + 1u) >> 1;
-        if (task_of(P, mid).groupBegin <= w) t = mid; else hi = mid - 1u;
+        if (task_of(P, mid).*begin <= w) t = mid; else hi = mid - 1u;
     }
     return t;
 }
 
-// Every warp takes a run of consecutive groups of four results (columns of B, then rows of A, so that
-// most columns are final when a row looks its match's up), eight lanes a result.
+// Every warp takes a run of consecutive groups of four results (columns of B, then rows of A), eight
+// lanes a result.
 //
-// A row's cross-check bit needs the final index of its match's column, which another warp may not have
+// kFlags: it sets the rows' flags too. A row's cross-check bit needs the final index of its match's column, which another warp may not have
 // written yet. It is decided from either state: the column's distance must be the row's; then its
 // index is the row itself (also as a chunk's first index: no earlier row of that chunk), or another
 // row, or the first index of the row's own chunk - and in that last case the row is the column's match
-// exactly if no earlier row of the chunk is as close. The alternatives: a grid-wide barrier (one
-// cooperative launch for matching, resolution and flags) needs all its blocks resident at once, which
-// a green context or a long kernel on another stream does not give (600 x 600, one call alone with all
-// outputs: 74 us, against 68 this way); a launch of its own for the flags costs 2 us in small
-// calls and re-reads the results in large ones (16384 x 16384 94 us against 90).
-template <int N>
+// exactly if no earlier row of the chunk is as close. The alternatives: a launch of its own for the
+// flags, which is better where there are many results (small_results); a grid-wide barrier (one
+// cooperative launch for matching, resolution and flags), which needs all its blocks resident at once:
+// a green context or a long kernel on another stream does not give that (and 600 x 600, one call alone
+// with all outputs, took 74 us, against 68 as three launches).
+template <int N, bool kFlags>
 __global__ void __launch_bounds__(256) bf_resolve_kernel(const __grid_constant__ Params<N> P) {
     const uint32_t lane = threadIdx.x & 31u, l8 = lane & 7u;
     const uint32_t warps = gridDim.x * 8u;
@@ -301,7 +302,7 @@ __global__ void __launch_bounds__(256) bf_resolve_kernel(const __grid_constant__
     const uint32_t first = (blockIdx.x * 8u + (threadIdx.x >> 5)) * run;
     if (first >= P.totalGroups) return;
     const uint32_t end = min(P.totalGroups, first + run);
-    uint32_t t = task_at(P, first);
+    uint32_t t = task_at(P, &TaskDev::groupBegin, first);
     grid_dep_wait();
     for (uint32_t w = first; w < end; ++w) {
         while (t + 1 < P.nTasks && task_of(P, t + 1).groupBegin <= w) ++t;
@@ -334,7 +335,7 @@ __global__ void __launch_bounds__(256) bf_resolve_kernel(const __grid_constant__
             if (s < old) T.secondA[i] = s;
             s = min(s, old);
         }
-        if (!T.flagsA) continue;
+        if (!kFlags) continue;
         const uint32_t j = at != ~0u ? at : j0, c0 = i & ~(kChunk - 1u);
         unsigned long long cb = row && j < T.nB ? __ldcg(&T.bestB[j]) : ~0ull;
         cb = __shfl_sync(0xffffffffu, cb, int(lane & 24u));  // one state of it for the eight lanes
@@ -353,6 +354,32 @@ __global__ void __launch_bounds__(256) bf_resolve_kernel(const __grid_constant__
             if (has && uint64_t(P.ratioDen) * d < uint64_t(P.ratioNum) * s) f |= 1u;
             T.flagsA[i] = f;
         }
+    }
+}
+
+// The flags as a launch of their own: bit0 ratio test, bit1 cross-check. Every warp takes a run of
+// 32-row groups.
+template <int N>
+__global__ void __launch_bounds__(256) bf_flags_kernel(const __grid_constant__ Params<N> P) {
+    const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * 8u;
+    const uint32_t run = (P.totalRowGroups + warps - 1u) / warps;
+    const uint32_t first = (blockIdx.x * 8u + (threadIdx.x >> 5)) * run;
+    if (first >= P.totalRowGroups) return;
+    const uint32_t end = min(P.totalRowGroups, first + run);
+    uint32_t t = task_at(P, &TaskDev::rowGroupBegin, first);
+    for (uint32_t w = first; w < end; ++w) {
+        while (t + 1 < P.nTasks && task_of(P, t + 1).rowGroupBegin <= w) ++t;
+        const TaskDev& T = task_of(P, t);
+        const uint32_t i = (w - T.rowGroupBegin) * 32u + lane;
+        if (i >= T.nA) continue;
+        const unsigned long long bm = __ldcg(&T.bestA[i]);
+        const uint32_t j = uint32_t(bm & 0xFFFFFFFFu), d = uint32_t(bm >> 32);
+        uint32_t f = 0;
+        if (j != ~0u) {
+            if (uint64_t(P.ratioDen) * d < uint64_t(P.ratioNum) * __ldcg(&T.secondA[i])) f |= 1u;
+            if (j < T.nB && uint32_t(__ldcg(&T.bestB[j]) & 0xFFFFFFFFu) == i) f |= 2u;
+        }
+        T.flagsA[i] = f;
     }
 }
 
@@ -772,6 +799,13 @@ static int launch(void (*kernel)(P), uint32_t grid, uint32_t threads, size_t sme
     return RSFM_OK;
 }
 
+// Up to four groups of results for each warp that fits on the device (4 blocks of 8 per SM), the
+// resolution starts while the matcher still runs, and sets the flags. Beyond, an early start leaves it
+// the matcher's small L1 and the flags' look-ups come while most columns are open; us with all outputs,
+// this way against waiting and a launch for the flags: 32768 x 32768 (16 K groups) 247.4 and 251.2, plan
+// of 16 pairs (26 K) 89.7 and 88.4, of 40 (100 K) 394 and 374, of 512 (2.3 M) 11860 and 11300.
+static bool small_results(const ParamsBase& P, int nsm) { return P.totalGroups <= uint32_t(nsm) * 128u; }
+
 // The matcher and what follows it. afterInit: the kernel before on the stream is this call's
 // initialisation (which waits for all before it, so the matcher may read its inputs at once).
 template <bool kSecond, int N>
@@ -783,10 +817,16 @@ static int launch_match(const Params<N>& P, int nsm, cudaStream_t stream, bool a
                         sizeof(Smem) + 1024, stream, afterInit, P);
         if (st != RSFM_OK) return st;
     }
-    if (P.totalGroups > 0)
-        return launch(bf_resolve_kernel<N>, std::min<uint32_t>((P.totalGroups + 7) / 8, uint32_t(nsm) * 64u), 256, 0, stream,
+    if (P.totalGroups == 0) return RSFM_OK;
+    const uint32_t grid = std::min<uint32_t>((P.totalGroups + 7) / 8, uint32_t(nsm) * 64u);
+    const bool small = small_results(P, nsm), flags = P.totalRowGroups > 0;
+    if (small)
+        return launch(flags ? bf_resolve_kernel<N, true> : bf_resolve_kernel<N, false>, grid, 256, 0, stream,
                       P.totalUnits > 0, P);
-    return RSFM_OK;
+    const int st = launch(bf_resolve_kernel<N, false>, grid, 256, 0, stream, false, P);
+    if (st != RSFM_OK || !flags) return st;
+    return launch(bf_flags_kernel<N>, std::min<uint32_t>((P.totalRowGroups + 7) / 8, uint32_t(nsm) * 64u), 256, 0, stream,
+                  false, P);
 }
 
 // Fills a task's device description and counts it into P's totals. Empty sides get no units, and of
@@ -805,6 +845,8 @@ static int fill_task(TaskDev* T, const rsfm_sift_bf_task& in, uint32_t* second, 
     T->unitBegin = P->totalUnits;
     T->groupBegin = P->totalGroups;
     T->rowBlocks = 1;
+    T->rowGroupBegin = P->totalRowGroups;
+    if (flags) P->totalRowGroups += (T->nA + 31) / 32;
     if (T->nA > 0 && (T->nB > 0 || flags)) P->totalGroups += uint32_t((uint64_t(T->nA) + T->nB + 3) / 4);
     if (T->nA == 0 || T->nB == 0) return RSFM_OK;
     int st = encode_desc_tmap(&T->tmA, in.descA, T->nA, kUnitRows);
