@@ -213,13 +213,15 @@ def test_user_graph_capture_and_streams(rsfm, oracle):
         _check(oracle, a, b, got)
 
 
-@pytest.mark.parametrize("na,nb", [(64, 20000), (20000, 64), (1, 5000), (5000, 1)])
+@pytest.mark.parametrize("na,nb", [(64, 20000), (20000, 64), (1, 5000), (5000, 1), (75400, 300), (75600, 300), (300, 75600)])
 def test_few_blocks_many_results(rsfm, oracle, na, nb):
-    # Long thin pairs: little matching, many results, and no launch more than a square pair's.
+    # Long thin pairs: little matching, many results, and no launch more than a square pair's. The flags
+    # are a launch of their own only beyond 128 groups of four results per SM.
     a, b = synth.make_pair(na, nb, 0.5, 8.0, seed=na + 2 * nb)[:2]
     task = rsfm.BFTask(_dev(a), _dev(b))
     rsfm.bf_match_ext([task])
-    assert rsfm.last_launch_count() == 3
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert rsfm.last_launch_count() == (3 if (na + nb + 3) // 4 <= 128 * sms else 4)
     _check(oracle, a, b, _run_ext(rsfm, [(a, b)])[0])
 
 
