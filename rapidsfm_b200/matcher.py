@@ -27,8 +27,8 @@ RATIO_DEN_08 = 100
 
 
 def _stream_ptr(stream):
-    if stream is None:
-        stream = torch.cuda.current_stream()
+    if stream is None:  # (torch.cuda.current_stream() builds an object: 3.4 us, three times in a small pair's call of 45)
+        return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
     return ctypes.c_void_p(stream.cuda_stream)
 
 

@@ -311,3 +311,14 @@ def test_calls_whose_kernels_overlap(rsfm, oracle):
             np.testing.assert_array_equal(np.stack(rsfm.unpack_best(t.bestB), 1), g)
         np.testing.assert_array_equal(ext.secondA.cpu().numpy().view(np.uint32), sec)
         np.testing.assert_array_equal(ext.flagsA.cpu().numpy().view(np.uint32), flags)
+
+
+def test_default_stream_is_the_current_one(rsfm):
+    # Without a stream argument a call goes to torch's current stream of the current device.
+    from rapidsfm_b200.matcher import _stream_ptr
+    assert _stream_ptr(None).value == (torch.cuda.current_stream().cuda_stream or None)
+    for priority in (0, -1):
+        s = torch.cuda.Stream(priority=priority)
+        with torch.cuda.stream(s):
+            assert _stream_ptr(None).value == s.cuda_stream == _stream_ptr(s).value
+    assert _stream_ptr(None).value == (torch.cuda.current_stream().cuda_stream or None)
