@@ -20,7 +20,12 @@ namespace {
 
 std::mutex g_cache_lock;
 
-// Device SM count, pair count (log2) and log2 histograms of the A and B sizes.
+// Version of the matcher that the cached choices and times belong to: raised whenever its units, its
+// phases or the meaning of an option change. Lines of another version are not answers (lines without
+// one are from before the 256 x 256 units).
+constexpr int kMatcherVersion = 2;
+
+// Matcher version, device SM count, pair count (log2) and log2 histograms of the A and B sizes.
 std::string signature(const rsfm_sift_bf_task* tasks, size_t n) {
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
@@ -31,7 +36,7 @@ std::string signature(const rsfm_sift_bf_task* tasks, size_t n) {
         hb[tasks[t].nbDescB ? 32 - __builtin_clz(tasks[t].nbDescB) : 0]++;
     }
     std::ostringstream os;
-    os << "sm" << nsm << ":n" << (n ? 64 - __builtin_clzll(uint64_t(n)) : 0) << ":a";
+    os << "v" << kMatcherVersion << ":sm" << nsm << ":n" << (n ? 64 - __builtin_clzll(uint64_t(n)) : 0) << ":a";
     for (int i = 0; i < 33; ++i)
         if (ha[i]) os << i << "x" << (32 - __builtin_clz(uint32_t(ha[i]))) << ",";
     os << ":b";

@@ -105,6 +105,22 @@ def test_autotune_and_cache(rsfm, oracle, tmp_path):
     plan.close()
 
 
+def test_autotune_cache_of_another_build(rsfm, tmp_path):
+    """A cache line written before the signature carried the kernel's version is not an answer for this
+    kernel: the batch is timed again and gets a line of its own."""
+    pairs = _pairs(3, 200, 900, 18)
+    tasks = [rsfm.BFTask(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()) for a, b in pairs]
+    cache = tmp_path / "bf_tune.txt"
+    rsfm.autotune_plan(tasks, cache_path=str(cache), reps=1)
+    sig = cache.read_text().split()[0]
+    old = sig[sig.index("sm"):]  # "sm<count>:n...", as it was
+    cache.write_text(old + " 2 8 2 1 0.0000001\n")
+    _, ms = rsfm.autotune_plan(tasks, cache_path=str(cache), reps=1)
+    assert ms > 0.001
+    lines = cache.read_text().splitlines()
+    assert len(lines) == 2 and lines[1].split()[0] == sig != old
+
+
 def test_plan_batched_workload_sizes(rsfm, oracle):
     """The batched workload at its own sizes: 64 seeded pairs with N, M ~ U[2000, 16000],
     overlap ~ U[0.1, 0.7], noise ~ U[4, 12], through the autotuned graph plan; every output of
