@@ -20,22 +20,41 @@ void set_last_cuda_error(cudaError_t e, const char* where) {
 void launch_count_reset() { t_launches = 0; }
 void launch_count_add(uint32_t n) { t_launches += n; }
 
-// One word per device, written by kernels when a bounded wait gives up.
+// One word per device context, written by kernels when a bounded wait gives up.
 __device__ uint32_t g_device_error = 0;
 
-// Per-device facts that every call needs: looked up once (a small call is bound by its host time).
+// Facts that every call needs are looked up once (a small call is bound by its host time): what belongs
+// to the device by its number, what belongs to its context by the context's id, which no other context
+// of the process ever has (a second context of the device, or the one after a device reset, has this
+// library's variables elsewhere and its kernels' attributes unset).
 constexpr int kMaxDevices = 64;
 
+// Id of the current context; 0 when there is none yet or the driver does not say.
+static unsigned long long context_id() {
+    using Fn = CUresult (*)(CUcontext, unsigned long long*);
+    static const Fn fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return reinterpret_cast<Fn>(p);
+    }();
+    unsigned long long id = 0;
+    return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
 uint32_t* device_error_word() {
-    static std::atomic<uint32_t*> words[kMaxDevices];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-    if (dev >= 0 && dev < kMaxDevices)
-        if (uint32_t* w = words[dev].load(std::memory_order_acquire)) return w;
+    static thread_local struct {
+        unsigned long long id;
+        uint32_t* word;
+    } last = {0, nullptr};
+    const unsigned long long id = context_id();
+    if (id != 0 && id == last.id) return last.word;
     void* p = nullptr;
     if (cudaGetSymbolAddress(&p, g_device_error) != cudaSuccess) return nullptr;
-    if (dev >= 0 && dev < kMaxDevices) words[dev].store(static_cast<uint32_t*>(p), std::memory_order_release);
-    return static_cast<uint32_t*>(p);
+    last = {context_id(), static_cast<uint32_t*>(p)};
+    return last.word;
 }
 
 static PFN_cuTensorMapEncodeTiled_v12000 get_encode_fn() {
@@ -165,14 +184,13 @@ extern "C" const char* rsfm_last_cuda_error(void) { return t_last_error; }
 namespace rsfm_b200 {
 
 int set_max_dynamic_smem(const void* kernel, size_t bytes) {
-    int dev = 0;
-    RSFM_CUDA_TRY(cudaGetDevice(&dev));
     static std::mutex mu;
-    static std::set<std::pair<const void*, int>> done;
+    static std::set<std::pair<const void*, unsigned long long>> done;  // (kernel, context)
+    const unsigned long long id = context_id();
     std::lock_guard<std::mutex> lk(mu);
-    if (done.count({kernel, dev})) return RSFM_OK;
+    if (id != 0 && done.count({kernel, id})) return RSFM_OK;
     RSFM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-    done.insert({kernel, dev});
+    if (id != 0) done.insert({kernel, id});
     return RSFM_OK;
 }
 

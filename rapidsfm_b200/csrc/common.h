@@ -42,8 +42,8 @@ int encode_bf16_tmap(CUtensorMap* out, const void* base, uint64_t rows, uint64_t
                      uint32_t boxRows);
 
 int sm_count();
-// Raises a kernel's dynamic shared-memory limit on the current device, once per (kernel, device):
-// the attribute belongs to the device's context, so a process using several GPUs sets it on each.
+// Raises a kernel's dynamic shared-memory limit in the current context, once per (kernel, context):
+// a process using several GPUs, or several contexts on one, sets it in each.
 int set_max_dynamic_smem(const void* kernel, size_t bytes);
 // Stream-ordered scratch pool of this library on the current device (keeps its memory).
 int scratch_pool(cudaMemPool_t* pool);
@@ -53,7 +53,7 @@ int scratch_pool(cudaMemPool_t* pool);
 bool profile_begin(cudaStream_t s, void** token);
 void profile_end(cudaStream_t s, void* token);
 
-// Address of this library's device-side error word on the current device.
+// Address of this library's device-side error word in the current context.
 uint32_t* device_error_word();
 
 }  // namespace rsfm_b200

@@ -322,3 +322,38 @@ def test_default_stream_is_the_current_one(rsfm):
         with torch.cuda.stream(s):
             assert _stream_ptr(None).value == s.cuda_stream == _stream_ptr(s).value
     assert _stream_ptr(None).value == (torch.cuda.current_stream().cuda_stream or None)
+
+
+def test_second_context_of_the_device(rsfm, oracle):
+    """What the library keeps between calls belongs to a context: after calls in the primary one, a
+    call in another context of the same device uses that context's variables and kernel attributes."""
+    cu = pytest.importorskip("cuda.bindings.driver")
+
+    def ok(r):
+        assert r[0] == cu.CUresult.CUDA_SUCCESS, r[0]
+        return r[1] if len(r) == 2 else None
+
+    a, b = synth.make_pair(700, 900, 0.5, 8.0, seed=91)[:2]
+    _check(oracle, a, b, _run_ext(rsfm, [(a, b)])[0])  # (primary context)
+    lib = rsfm._lib.load()
+    efwd, ebwd, _ = oracle.bf_match(a, b)
+    ctx = ok(cu.cuCtxCreate(0, ok(cu.cuDeviceGet(torch.cuda.current_device()))))
+    try:
+        bufs = []
+        for x in (a, b, oracle.sqr_norm(a), oracle.sqr_norm(b), np.zeros((len(a), 2), np.uint32), np.zeros((len(b), 2), np.uint32)):
+            x = np.ascontiguousarray(x)
+            p = ok(cu.cuMemAlloc(x.nbytes))
+            ok(cu.cuMemcpyHtoD(p, x.ctypes.data, x.nbytes))
+            bufs.append((int(p), x))
+        (pa, _), (pb, _), (na, _), (nb, _), (ra, fwd), (rb, bwd) = bufs
+        task = (rsfm._lib.SiftBFTask * 1)(rsfm._lib.SiftBFTask(len(a), len(b), pa, pb, ra, rb, na, nb))
+        rsfm._lib.check(lib.rsfm_bf_match(task, 1, None), "rsfm_bf_match")
+        assert rsfm.device_error() == 0
+        ok(cu.cuCtxSynchronize())
+        ok(cu.cuMemcpyDtoH(fwd.ctypes.data, ra, fwd.nbytes))
+        ok(cu.cuMemcpyDtoH(bwd.ctypes.data, rb, bwd.nbytes))
+    finally:
+        ok(cu.cuCtxDestroy(ctx))
+    np.testing.assert_array_equal(fwd, efwd)
+    np.testing.assert_array_equal(bwd, ebwd)
+    _check(oracle, a, b, _run_ext(rsfm, [(a, b)])[0])  # (the primary one again)
