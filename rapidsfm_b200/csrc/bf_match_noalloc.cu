@@ -5,7 +5,6 @@
 // enqueuing anything.
 #include "bf_internal.h"
 #include "common.h"
-#include <algorithm>
 
 namespace rsfm_b200 {
 namespace noalloc {
@@ -17,16 +16,12 @@ using namespace rsfm_b200;
 
 extern "C" int rsfm_bf_match_noalloc(const rsfm_sift_bf_task* tasks, size_t nbTasks, cudaStream_t stream) {
     launch_count_reset();
-    // The same argument checks as rsfm_bf_match, then the limit on the total query rows.
+    // The same argument checks as rsfm_bf_match, then the limit on the total query rows, which callers may
+    // rely on (rsfm_bf_match itself allocates nothing and has no such limit).
     int st = bf::validate(tasks, nbTasks);
     if (st != RSFM_OK) return st;
     size_t total = 0;
     for (size_t t = 0; t < nbTasks; ++t) total += tasks[t].nbDescA;
     if (total > noalloc::kNoAllocMaxRows) return RSFM_ERR_CAPACITY;
-    for (size_t i = 0; i < nbTasks; i += bf::kMaxTasksPerLaunch) {
-        const size_t n = std::min<size_t>(bf::kMaxTasksPerLaunch, nbTasks - i);
-        st = bf::launch_chunk(tasks + i, n, nullptr, nullptr, 0, 1, stream);
-        if (st != RSFM_OK) return st;
-    }
-    return RSFM_OK;
+    return rsfm_bf_match(tasks, nbTasks, stream);
 }

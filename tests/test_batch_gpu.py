@@ -27,7 +27,7 @@ def _res(rsfm, t):
 
 
 @pytest.mark.parametrize("graph", [True, False])
-@pytest.mark.parametrize("groups", [2, 4])
+@pytest.mark.parametrize("groups", [2, 4])  # (accepted, without effect)
 def test_plan_equals_per_pair(rsfm, oracle, graph, groups):
     pairs = _pairs(37, 100, 2500, 5)
     tasks = [rsfm.BFTask(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()) for a, b in pairs]
@@ -82,7 +82,8 @@ def test_autotune_and_cache(rsfm, oracle, tmp_path):
     tasks = [rsfm.BFTask(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()) for a, b in pairs]
     cache = str(tmp_path / "bf_tune.txt")
     opts, ms = rsfm.autotune_plan(tasks, cache_path=cache, reps=2)
-    assert opts.rowTiles in (2, 4, 8) and opts.colBlocks in (1, 2, 4, 8) and opts.epilogueGroups in (2, 4)
+    # one of the five unit lengths that the tuner times
+    assert (opts.rowTiles, opts.colBlocks) in ((8, 8), (8, 4), (8, 2), (8, 1), (4, 1)) and opts.schedule in (0, 1)
     assert ms > 0
     assert len(open(cache).read().splitlines()) == 1
     # the same kind of batch is answered from the cache, without timing

@@ -169,7 +169,7 @@ def test_unit_and_chunk_edges(rsfm, oracle, na, nb, seed):
 
 @pytest.mark.parametrize("sizes", [[(700, 900), (300, 0), (0, 40), (1000, 20)], [(9000, 9100), (30, 8000)]])
 def test_phases_in_one_launch_and_apart(rsfm, oracle, sizes):
-    # A call is init, match and resolution with flags, whatever its size. Same results from both entry
+    # A call is init, match and resolution, with the flags in it. Same results from both entry
     # points, empty sides.
     pairs = []
     for k, (na, nb) in enumerate(sizes):
@@ -190,7 +190,7 @@ def test_phases_in_one_launch_and_apart(rsfm, oracle, sizes):
 
 
 def test_user_graph_capture_and_streams(rsfm, oracle):
-    # A caller's own graph around a small (cooperative) call, and calls on two streams at once.
+    # A caller's own graph around a small call (launches that overlap), and calls on two streams at once.
     pairs = [synth.make_pair(800, 1000, 0.5, 8.0, seed=40)[:2], synth.make_pair(1200, 600, 0.5, 8.0, seed=41)[:2]]
     tasks = [rsfm.BFTask(_dev(a), _dev(b)) for a, b in pairs]
     rsfm.bf_match_ext(tasks)
@@ -198,7 +198,9 @@ def test_user_graph_capture_and_streams(rsfm, oracle):
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
         rsfm.bf_match_ext([tasks[0]])
-    tasks[0].bestA.fill_(0)
+    for t in tasks:  # all that the replays and the direct calls have to write
+        for out in (t.bestA, t.bestB, t.secondA, t.flagsA):
+            out.fill_(0x55)
     torch.cuda.synchronize()
     streams = [torch.cuda.Stream() for _ in range(2)]
     for _ in range(5):
