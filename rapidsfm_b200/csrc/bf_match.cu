@@ -24,14 +24,16 @@
 // The epilogue keeps, per lane, only maxima of 16-column chunks: one key (value << 8 | chunk
 // code) per chunk, the best (and for the second-best output the two best) in registers. Results
 // are published as (distance, first index of the chunk), the minimum over chunks being the
-// lexicographic (distance, chunk) minimum; a last phase (resolve_item) then finds the index inside the
-// winning chunk, and the second-best inside it, from 16 exact distances.
+// lexicographic (distance, chunk) minimum; bf_resolve_kernel then finds the index inside the winning
+// chunk, and the second-best inside it, from 16 exact distances.
 //
-// What bounds it: the tensor pipe. At 32768 x 32768 the two products take 2 x 5 K steps of 138
-// cycles per 128 x 256 values = 155 us on 148 SMs; keys formed on the CUDA cores instead (two
+// What bounds it: the tensor pipe. At 32768 x 32768 the two products take 2 x 5 K steps of 128
+// cycles per 128 x 256 values = 145 us on 148 SMs; a call with norms at hand takes 230 us there (at 16384
+// the tensor pipe is busy for 60 % of the matcher's cycles). Keys formed on the CUDA cores instead (two
 // multiply-adds and a trigger per distance, the design before this one) took 362 us at 53 % issue.
+// Where every unit holds a byte above 127, 9 K steps instead of 5, 260 us: 302 us at 32768 x 32768.
 //
-// Work decomposition. A "unit" is a block of 256 A rows times up to 32 blocks of 256 B columns.
+// Work decomposition. A "unit" is a block of 256 A rows times up to 16 blocks of 256 B columns.
 // Persistent CTAs take units round-robin. Per CTA (768 threads):
 //   warp 0      UMMA issuer (one thread; warp 1 owns the TMEM allocation, 2 and 3 are idle): per B
 //               block the tiles of both 128-row halves and the transposes of both 128-column
@@ -425,7 +427,9 @@ __global__ void __launch_bounds__(kThreads, 1) bf_match_kernel(const __grid_cons
     const uint32_t tmem = S.tmemBase;
     uint32_t* err = P.err;
 
-    // Registers: 768 threads x 80 at launch = 40 + 56 + 4 x 96 per thread of the six warpgroups.
+    // Registers: every one of the 768 threads has 80. Handing some of the issuer's and the preparation's
+    // to the epilogue (setmaxnreg, 88 or 96 there) ended in spills or moves: 251 to 287 us at
+    // 32768 x 32768 against 224.
     if (warp < 4) {
         // ------------------------------------------------------------ UMMA issuer
         // One thread, so that products complete in order (with two or four issuers their UMMAs take
